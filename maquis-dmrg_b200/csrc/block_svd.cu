@@ -234,11 +234,16 @@ __global__ void __launch_bounds__(SVD_THREADS) block_svd_jacobi(const SvdBlock* 
         if (lane == 0) sig[j] = sqrt(ss);
     }
     __syncthreads();
-    // descending order, ties by column index
+    // descending order, ties by column index, NaN (from a non-finite block) first: a total
+    // order, so that every entry of rank_col is written
     for (uint32_t j = threadIdx.x; j < n; j += blockDim.x) {
         const double sj = sig[j];
         uint32_t rk = 0;
-        for (uint32_t i = 0; i < n; ++i) rk += (sig[i] > sj || (sig[i] == sj && i < j)) ? 1u : 0u;
+        for (uint32_t i = 0; i < n; ++i) {
+            const double si = sig[i];
+            const bool same = si == sj || (isnan(si) && isnan(sj));
+            rk += (si > sj || (isnan(si) && !isnan(sj)) || (same && i < j)) ? 1u : 0u;
+        }
         rank_col[rk] = int(j);
     }
     __syncthreads();
