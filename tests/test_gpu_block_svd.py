@@ -79,6 +79,58 @@ def test_block_svd_graded_rank_deficient_and_zero_blocks():
         assert np.linalg.norm(U @ np.diag(s) @ Vt - a) <= TOL * np.linalg.norm(a)
 
 
+# sizes around the register and cluster classes (32 elements per lane slot; 16 column pairs
+# per CTA, 1, 2, 4 or 8 CTAs; above 256 rows the general kernel), square and not
+EDGES = [(31, 31), (32, 32), (33, 33), (64, 63), (63, 64), (65, 65), (128, 127), (129, 128), (128, 129), (130, 33),
+         (256, 255), (255, 256), (256, 256), (256, 2), (2, 256), (256, 1), (257, 40), (40, 257)]
+
+
+@pytest.mark.parametrize("decades", [0, 8, 14])
+def test_block_svd_class_edges(decades):
+    """Singular values falling by `decades`: reconstruction, orthogonality of both factors
+    (also of the directions of small singular values) and singular values."""
+    rng = np.random.default_rng(7)
+    mats = []
+    for r, c in EDGES:
+        k = min(r, c)
+        w = 10.0 ** (-decades * np.arange(k) / max(k, 1))
+        mats.append((np.linalg.qr(rng.standard_normal((r, k)))[0] * w) @ np.linalg.qr(rng.standard_normal((c, k)))[0].T)
+    for a, (U, s, Vt) in zip(mats, _svd_dev(mats)):
+        _check(a, U, s, Vt)
+        assert np.max(np.abs(U.T @ U - np.eye(U.shape[1]))) <= TOL
+
+
+def test_block_svd_column_scaling_keeps_small_values():
+    """A = B diag(d) with B well conditioned and d over 40 decades: one-sided Jacobi gives the
+    small singular values to relative accuracy (here within 1e-10: the condition of the
+    random B, at most a few thousand, times rounding), also after the pivoted QR."""
+    rng = np.random.default_rng(8)
+    mats, refs = [], []
+    for n in (24, 70, 150):
+        q = np.linalg.qr(rng.standard_normal((n, n)))[0]
+        d = 10.0 ** (-40.0 * np.arange(n) / n)
+        mats.append(q * d[rng.permutation(n)])  # orthogonal columns: the singular values are d
+        refs.append(d)
+    for a, d, (U, s, Vt) in zip(mats, refs, _svd_dev(mats)):
+        assert np.max(np.abs(s / d - 1.0)) <= 1e-10
+
+
+def test_block_svd_zero_columns_and_non_finite_blocks_take_the_general_kernel():
+    """Exactly zero columns: zero singular values with zero U columns and an orthonormal V;
+    a block with a NaN gives NaN and leaves the other blocks alone."""
+    rng = np.random.default_rng(9)
+    a = rng.standard_normal((90, 80))
+    a[:, ::3] = 0.0
+    bad = rng.standard_normal((40, 40))
+    bad[3, 5] = np.nan
+    c = rng.standard_normal((70, 70))
+    (U, s, Vt), (Ub, sb, Vb), good = _svd_dev([a, bad, c])
+    _check(a, U, s, Vt)
+    assert np.all(U[:, s == 0.0] == 0.0) and np.sum(s == 0.0) >= 1
+    assert np.any(np.isnan(sb)) or np.any(np.isnan(Ub)) or np.any(np.isnan(Vb))
+    _check(c, *good)
+
+
 def test_block_svd_rejects_null_blocks():
     rows = np.array([2], dtype=np.uint32)
     nul = (capi.C.c_void_p * 1)(None)
