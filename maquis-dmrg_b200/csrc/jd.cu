@@ -229,8 +229,11 @@ dmrgb200_status dmrgb200::solve_stepwise(dmrgb200_plan_t plan, uint64_t n, const
     if (max_iter < 1 || max_iter > 32) return noalloc_fail(DMRGB200_INVALID_ARGUMENT, "max_iter must be in 1..32");
     if (n_ortho > 8) return noalloc_fail(DMRGB200_INVALID_ARGUMENT, "at most 8 orthogonal vectors");
     cudaStream_t st = static_cast<cudaStream_t>(cuda_stream);
-    if (plan_solver_mode(plan) == DMRGB200_SOLVER_GRAPH)
-        return solve_graph(plan, plan_jd_cache(plan), n, x0, ortho, n_ortho, tol, max_iter, energy, x_out, stats, st);
+    if (plan_solver_mode(plan) == DMRGB200_SOLVER_GRAPH) {
+        const dmrgb200_status gs =
+            solve_graph(plan, plan_jd_cache(plan), n, x0, ortho, n_ortho, tol, max_iter, energy, x_out, stats, st);
+        if (gs != DMRGB200_NOT_SUPPORTED) return gs;
+    }
     const int nv = int(2 * max_iter + 2 + n_ortho);
     Workspace w;
     cudaError_t e;

@@ -1,18 +1,26 @@
 // Jacobi-Davidson as one CUDA graph: every scalar of the iteration lives on the
-// device, one iteration is the body of a conditional WHILE node, and the body's
-// last reduction decides whether it runs again.  The steps are those of the
-// stepwise solver in jd.cu (ietl/jacobi.h:386-474, ietl_jacobi_davidson.h:35-76):
-// MGS with one refinement pass below kappa = 0.25, projection of the
-// orthogonal vectors, Rayleigh-Ritz (cyclic Jacobi on the k x k projected
-// matrix, here by one warp), convergence |r| <= tol |theta| or |r| < tol, and
-// the correction t = -r + (r.u / u.u) u.
+// device, one iteration is the body of a conditional WHILE node (one H psi and one
+// jd_step launch), and the step decides whether the body runs again.  The steps are
+// those of the stepwise solver in jd.cu (ietl/jacobi.h:386-474,
+// ietl_jacobi_davidson.h:35-76): MGS with one refinement pass below kappa = 0.25,
+// projection of the orthogonal vectors, Rayleigh-Ritz (cyclic Jacobi on the k x k
+// projected matrix), convergence |r| <= tol |theta| or |r| < tol, and the correction
+// t = -r + (r.u / u.u) u.
 //
-// Reductions: every vector kernel runs on a fixed grid; each block reduces its
-// slice in a fixed order and the last block to arrive sums the block partials
-// in block order, so a solve is bitwise reproducible.  Each body sets the WHILE
-// condition to 0 first and only the residual kernel sets it back to 1, after
-// incrementing the iteration count, so the loop ends after at most max_iter
-// bodies whatever the data.
+// jd_step is one cooperative launch of one CTA per SM.  Every thread owns the same
+// elements of all vectors throughout and keeps the target (t, u, uA) in registers; what
+// the CTAs exchange are the inner products: each CTA publishes its partial sums, a grid
+// barrier follows, and every CTA adds all partials in the same order, so all hold the
+// same coefficients without a second exchange, and a solve is bitwise reproducible.
+// What bounds it are those barriers (iteration k has k + 4 of them, 2k + 5 with
+// refinement) and the chain of rotations of the k x k eigenproblem, which every CTA
+// solves for itself; as separate launches, one per inner product and vector operation
+// (about 30 per iteration), it was the launches and their drains.
+//
+// Each body sets the WHILE condition to 0 first and sets it back to 1 only at its end,
+// after incrementing the iteration count, so the loop ends after at most max_iter bodies
+// whatever the data.  The wait at a grid barrier is bounded (2 s): a CTA that gives up
+// records it, every later step returns at once and the solve reports DMRGB200_TIMEOUT.
 #include <cuda_runtime.h>
 
 #include <cmath>
@@ -20,6 +28,7 @@
 #include <vector>
 
 #include "../../include/dmrgb200.h"
+#include "async_copy.cuh"
 #include "device.hpp"
 
 namespace dmrgb200 {
@@ -30,29 +39,26 @@ cudaError_t plan_ensure_tuned(dmrgb200_plan_t plan, const double* x, double* y, 
 
 namespace {
 
-constexpr int JT = 256;        // threads per block of the vector kernels
-constexpr int MAXK = 32;       // max_iter bound
+constexpr int JT = 1024;       // threads per CTA of the step kernels (one CTA per SM)
+constexpr int MAXK = 32;       // max_iter bound (and the warps of a CTA)
 constexpr int MAXO = 8;        // orthogonal vectors bound
+constexpr int EPT = 4;         // elements per thread kept in registers
 
 struct JdState {
-    unsigned counter;
-    int iter, done, status, converged, refine;
-    double tau, tn, theta, rnorm, corr;
-    double c[2][MAXK];     // MGS coefficients, per pass
-    double pc[MAXO];       // projection coefficients of the current target
+    unsigned long long barrier;  // arrivals at grid barriers since the solve began
+    int iter, done, status, converged;  // status: 1 vanished direction, 2 barrier wait ran out
+    double theta, rnorm;
     double oo[MAXO];       // <o_i, o_i>
     double M[MAXK * MAXK]; // projected matrix, column-major, leading dimension MAXK
-    double s[MAXK];        // Ritz vector coefficients
 };
 
 struct JdArgs {
     double* vec;          // vector slots, n doubles each
     uint64_t n;
-    uint64_t chunk;       // elements per block
     int max_iter, n_ortho;
     double tol;
     JdState* st;
-    double* partial;      // per-block partial sums: MAXK + 2 rows of gridDim
+    double* partial;      // [2][MAXK][grid] partial sums of the CTAs
     cudaGraphConditionalHandle cond;
 };
 
@@ -65,346 +71,373 @@ __device__ __forceinline__ double* Tv(JdArgs const& a) { return a.vec + a.n * ui
 __device__ __forceinline__ double* Yv(JdArgs const& a) { return a.vec + a.n * uint64_t(2 * a.max_iter + 3); }
 __device__ __forceinline__ double* Ov(JdArgs const& a, int i) { return a.vec + a.n * uint64_t(2 * a.max_iter + 4 + i); }
 
-__device__ __forceinline__ uint64_t lo(JdArgs const& a) { return blockIdx.x * a.chunk; }
-__device__ __forceinline__ uint64_t hi(JdArgs const& a) {
-    uint64_t h = (blockIdx.x + 1) * a.chunk;
-    return h < a.n ? h : a.n;
-}
+// This thread's elements of one vector: registers (REG) or its own elements of a global
+// slot, which no other thread touches.
+template <bool REG>
+struct Own {
+    double r[REG ? EPT : 1];
+    double* g;
+    __device__ __forceinline__ double get(int e, uint64_t i) const { return REG ? r[e] : g[i]; }
+    __device__ __forceinline__ void set(int e, uint64_t i, double v) {
+        if (REG) r[e] = v;
+        else g[i] = v;
+    }
+};
 
-// block sum in a fixed order; the result is valid in thread 0
-__device__ double block_sum(double v) {
-    __shared__ double red[JT / 32];
+// f(e, i) for every element i this thread owns
+template <bool REG, class F>
+__device__ __forceinline__ void each(JdArgs const& a, F&& f) {
+    const uint64_t i0 = uint64_t(blockIdx.x) * JT + threadIdx.x, stride = uint64_t(gridDim.x) * JT;
+    if (REG) {
 #pragma unroll
-    for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
-    __syncthreads();
-    if ((threadIdx.x & 31) == 0) red[threadIdx.x >> 5] = v;
-    __syncthreads();
-    double s = 0.0;
-    if (threadIdx.x == 0)
-        for (int w = 0; w < JT / 32; ++w) s += red[w];
-    return s;
+        for (int e = 0; e < EPT; ++e) {
+            const uint64_t i = i0 + e * stride;
+            if (i < a.n) f(e, i);
+        }
+    } else {
+        for (uint64_t i = i0; i < a.n; i += stride) f(0, i);
+    }
 }
 
-// publish this block's partials and report whether it is the last block to arrive
-__device__ bool arrive(JdState* st) {
-    __shared__ int last;
+struct StepShared {
+    double red[JT / 32][MAXK];  // [warp][value]
+    double sum[MAXK];
+    double A[MAXK][MAXK + 1], Z[MAXK][MAXK + 1];
+    double s[MAXK];
+    double cs[MAXK / 2][2];
+    double theta;
+    int failed;
+};
+
+// Sums of nv per-thread values over the grid: warp trees, the CTA's partial sums to
+// global memory, a grid barrier, then warp w of every CTA adds value w over all CTAs (the
+// same order everywhere).  Results in sh.sum[0, nv).  `val(k, v)` gives the thread's values
+// k .. k + 3 (those below nv count), four at a time so that their loads overlap.  False when
+// the barrier's wait ran out.
+template <class F>
+__device__ bool grid_sums(JdArgs const& a, StepShared& sh, int nv, unsigned& phase, F&& val) {
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    double* part = a.partial + uint64_t(phase & 1u) * MAXK * gridDim.x;
+    ++phase;
+    for (int k = 0; k < nv; k += 4) {
+        double v[4] = {0.0, 0.0, 0.0, 0.0};
+        val(k, v);
+#pragma unroll
+        for (int o = 16; o > 0; o >>= 1)
+#pragma unroll
+            for (int j = 0; j < 4; ++j) v[j] += __shfl_xor_sync(0xffffffffu, v[j], o);
+        if (lane == 0)
+#pragma unroll
+            for (int j = 0; j < 4; ++j)
+                if (k + j < nv) sh.red[warp][k + j] = v[j];
+    }
+    __syncthreads();
+    if (warp < nv) {
+        double v = sh.red[lane][warp];
+#pragma unroll
+        for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
+        if (lane == 0) __stcg(part + uint64_t(warp) * gridDim.x + blockIdx.x, v);
+    }
     __syncthreads();
     if (threadIdx.x == 0) {
+        // arrive, then wait until every CTA of this generation has (each CTA arrives once per
+        // generation, so the arrival's number tells the generation)
         __threadfence();
-        last = atomicAdd(&st->counter, 1u) == gridDim.x - 1;
-    }
-    __syncthreads();
-    return last;
-}
-
-// sum of row r of the partial table over all blocks, by the whole (last) block:
-// every thread sums a fixed subset in order, then the fixed block tree; the
-// result is valid in thread 0
-__device__ double gather(JdArgs const& a, int r) {
-    double s = 0.0;
-    for (unsigned b = threadIdx.x; b < gridDim.x; b += JT) s += __ldcg(a.partial + uint64_t(r) * gridDim.x + b);
-    return block_sum(s);
-}
-
-__device__ void finish(JdArgs const& a) {
-    if (threadIdx.x == 0) a.st->counter = 0;
-}
-
-// dot of two slices
-__device__ double slice_dot(JdArgs const& a, const double* x, const double* y) {
-    double s = 0.0;
-    for (uint64_t i = lo(a) + threadIdx.x; i < hi(a); i += JT) s += x[i] * y[i];
-    return block_sum(s);
-}
-
-__global__ void __launch_bounds__(JT) jd_init(JdArgs a) {
-    if (blockIdx.x == 0 && threadIdx.x == 0) {
-        JdState* st = a.st;
-        st->counter = 0;
-        st->iter = st->done = st->status = st->converged = st->refine = 0;
-        st->tau = st->tn = st->theta = st->rnorm = st->corr = 0.0;
-    }
-}
-
-// <O(i), O(i)> into oo[i]
-__global__ void __launch_bounds__(JT) jd_oo(JdArgs a, int i) {
-    double p = slice_dot(a, Ov(a, i), Ov(a, i));
-    if (threadIdx.x == 0) a.partial[blockIdx.x] = p;
-    if (arrive(a.st)) {
-        const double g = gather(a, 0);
-        if (threadIdx.x == 0) a.st->oo[i] = g;
-        finish(a);
-    }
-}
-
-// target -= pc[i-1] O(i-1) (i > 0), then pc[i] = <O(i), target> / oo[i].
-// target: 0 = t, 1 = uA, 2 + j = O(j)
-__device__ double* target_of(JdArgs const& a, int target) {
-    return target == 0 ? Tv(a) : target == 1 ? UA(a) : Ov(a, target - 2);
-}
-__global__ void __launch_bounds__(JT) jd_proj(JdArgs a, int i, int target) {
-    double* x = target_of(a, target);
-    if (i > 0) {
-        const double c = a.st->pc[i - 1];
-        const double* o = Ov(a, i - 1);
-        for (uint64_t k = lo(a) + threadIdx.x; k < hi(a); k += JT) x[k] -= c * o[k];
-    }
-    double p = slice_dot(a, Ov(a, i), x);
-    if (threadIdx.x == 0) a.partial[blockIdx.x] = p;
-    if (arrive(a.st)) {
-        const double g = gather(a, 0);
-        if (threadIdx.x == 0) a.st->pc[i] = g / a.st->oo[i];
-        finish(a);
-    }
-}
-__global__ void __launch_bounds__(JT) jd_proj_close(JdArgs a, int last, int target) {
-    double* x = target_of(a, target);
-    const double c = a.st->pc[last];
-    const double* o = Ov(a, last);
-    for (uint64_t k = lo(a) + threadIdx.x; k < hi(a); k += JT) x[k] -= c * o[k];
-}
-
-// first kernel of an iteration: stop unless the residual kernel says otherwise; tau = |t|
-__global__ void __launch_bounds__(JT) jd_tau(JdArgs a) {
-    if (blockIdx.x == 0 && threadIdx.x == 0) cudaGraphSetConditional(a.cond, 0u);
-    double p = slice_dot(a, Tv(a), Tv(a));
-    if (threadIdx.x == 0) a.partial[blockIdx.x] = p;
-    if (arrive(a.st)) {
-        const double g = gather(a, 0);
-        if (threadIdx.x == 0) a.st->tau = sqrt(g);
-        finish(a);
-    }
-}
-
-// MGS step j of a pass: t -= c[pass][j-1] V(j-1), then c[pass][j] = <V(j), t>
-__global__ void __launch_bounds__(JT) jd_mgs(JdArgs a, int j, int pass) {
-    JdState* st = a.st;
-    if (j >= st->iter || (pass == 1 && !st->refine)) return;
-    double* t = Tv(a);
-    if (j > 0) {
-        const double c = st->c[pass][j - 1];
-        const double* v = V(a, j - 1);
-        for (uint64_t k = lo(a) + threadIdx.x; k < hi(a); k += JT) t[k] -= c * v[k];
-    }
-    double p = slice_dot(a, V(a, j), t);
-    if (threadIdx.x == 0) a.partial[blockIdx.x] = p;
-    if (arrive(st)) {
-        const double g = gather(a, 0);
-        if (threadIdx.x == 0) st->c[pass][j] = g;
-        finish(a);
-    }
-}
-
-// end of an MGS pass: apply the last coefficient; after pass 0 decide on refinement
-__global__ void __launch_bounds__(JT) jd_mgs_close(JdArgs a, int pass) {
-    JdState* st = a.st;
-    const int it = st->iter;
-    double* t = Tv(a);
-    const bool active = it > 0 && (pass == 0 || st->refine);
-    if (active) {
-        const double c = st->c[pass][it - 1];
-        const double* v = V(a, it - 1);
-        for (uint64_t k = lo(a) + threadIdx.x; k < hi(a); k += JT) t[k] -= c * v[k];
-    }
-    if (pass != 0) return;
-    double p = slice_dot(a, t, t);
-    if (threadIdx.x == 0) a.partial[blockIdx.x] = p;
-    if (arrive(st)) {
-        const double g = gather(a, 0);
-        if (threadIdx.x == 0) {
-            st->tn = sqrt(g);
-            st->refine = (it > 0 && st->tn < 0.25 * st->tau) ? 1 : 0;
-        }
-        finish(a);
-    }
-}
-
-// |t| after orthogonalisation; a vanished direction ends the solve
-__global__ void __launch_bounds__(JT) jd_tnorm(JdArgs a) {
-    double p = slice_dot(a, Tv(a), Tv(a));
-    if (threadIdx.x == 0) a.partial[blockIdx.x] = p;
-    if (arrive(a.st)) {
-        const double g = gather(a, 0);
-        if (threadIdx.x == 0) {
-            JdState* st = a.st;
-            st->tn = sqrt(g);
-            if (!(st->tn > 0.0)) {
-                st->status = 1;
-                st->done = 1;
+        const unsigned long long target = (atomicAdd(&a.st->barrier, 1ull) / gridDim.x + 1ull) * gridDim.x;
+        const unsigned long long t0 = async::global_ns();
+        unsigned long long seen;
+        sh.failed = 0;
+        for (;;) {
+            asm volatile("ld.acquire.gpu.u64 %0, [%1];" : "=l"(seen) : "l"(&a.st->barrier) : "memory");
+            if (seen >= target) break;
+            if (async::global_ns() - t0 > async::WAIT_LIMIT_NS) {
+                sh.failed = 1;
+                atomicExch(&a.st->status, 2);
+                break;
             }
         }
-        finish(a);
     }
+    __syncthreads();
+    if (sh.failed) return false;
+    if (warp < nv) {
+        double v = 0.0;
+        for (unsigned b = lane; b < gridDim.x; b += 32) v += __ldcg(part + uint64_t(warp) * gridDim.x + b);
+#pragma unroll
+        for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
+        if (lane == 0) sh.sum[warp] = v;
+    }
+    __syncthreads();
+    return true;
 }
 
-// t /= |t|; V(iter) = t
-__global__ void __launch_bounds__(JT) jd_store(JdArgs a) {
-    JdState* st = a.st;
-    const double inv = st->status ? 0.0 : 1.0 / st->tn;
-    double* t = Tv(a);
-    double* v = V(a, st->iter);
-    for (uint64_t k = lo(a) + threadIdx.x; k < hi(a); k += JT) {
-        double x = t[k] * inv;
-        t[k] = x;
+// Project the orthogonal vectors out of x: x -= <o_i, x> / <o_i, o_i> o_i in turn.
+template <bool REG>
+__device__ bool project(JdArgs const& a, StepShared& sh, unsigned& phase, Own<REG>& x, int no) {
+    for (int i = 0; i < no; ++i) {
+        const double* o = Ov(a, i);
+        double p = 0.0;
+        each<REG>(a, [&](int e, uint64_t k) { p += o[k] * x.get(e, k); });
+        if (!grid_sums(a, sh, 1, phase, [&](int, double* v) { v[0] = p; })) return false;
+        const double c = sh.sum[0] / a.st->oo[i];
+        each<REG>(a, [&](int e, uint64_t k) { x.set(e, k, x.get(e, k) - c * o[k]); });
+    }
+    return true;
+}
+
+// Basis vector V(it) from the target t: MGS against V(0..it), refinement, projection,
+// normalisation; also left in the H psi input.
+template <bool REG>
+__device__ bool basis_vector(JdArgs const& a, StepShared& sh, unsigned& phase, Own<REG>& t, int it) {
+    // tau^2 = <t, t> and the first coefficient in one exchange
+    double tt = 0.0, p = 0.0;
+    each<REG>(a, [&](int e, uint64_t k) {
+        const double x = t.get(e, k);
+        tt += x * x;
+        if (it > 0) p += V(a, 0)[k] * x;
+    });
+    if (!grid_sums(a, sh, it > 0 ? 2 : 1, phase, [&](int, double* v) {
+            v[0] = tt;
+            v[1] = p;
+        })) return false;
+    const double tau = sqrt(sh.sum[0]);
+    double nn = sh.sum[0], c = it > 0 ? sh.sum[1] : 0.0;
+    for (int pass = 0; it > 0 && pass < 2; ++pass) {
+        if (pass == 1) {
+            if (!(sqrt(nn) < 0.25 * tau)) break;
+            p = 0.0;
+            each<REG>(a, [&](int e, uint64_t k) { p += V(a, 0)[k] * t.get(e, k); });
+            if (!grid_sums(a, sh, 1, phase, [&](int, double* v) { v[0] = p; })) return false;
+            c = sh.sum[0];
+        }
+        // t -= c V(j) and, in the same pass over t, the next coefficient (or |t|^2 at the end)
+        for (int j = 0; j < it; ++j) {
+            const double* v = V(a, j);
+            const double* w = j + 1 < it ? V(a, j + 1) : nullptr;
+            p = 0.0;
+            each<REG>(a, [&](int e, uint64_t k) {
+                const double x = t.get(e, k) - c * v[k];
+                t.set(e, k, x);
+                p += (w ? w[k] : x) * x;
+            });
+            if (!grid_sums(a, sh, 1, phase, [&](int, double* v) { v[0] = p; })) return false;
+            c = nn = sh.sum[0];
+        }
+    }
+    if (a.n_ortho > 0) {
+        if (!project<REG>(a, sh, phase, t, a.n_ortho)) return false;
+        p = 0.0;
+        each<REG>(a, [&](int e, uint64_t k) { p += t.get(e, k) * t.get(e, k); });
+        if (!grid_sums(a, sh, 1, phase, [&](int, double* v) { v[0] = p; })) return false;
+        nn = sh.sum[0];
+    }
+    const double tn = sqrt(nn);
+    const bool vanished = !(tn > 0.0);
+    if (vanished && blockIdx.x == 0 && threadIdx.x == 0) {
+        a.st->status = 1;
+        a.st->done = 1;
+    }
+    const double inv = vanished ? 0.0 : 1.0 / tn;
+    double *in = Tv(a), *v = V(a, it);
+    each<REG>(a, [&](int e, uint64_t k) {
+        const double x = t.get(e, k) * inv;
+        in[k] = x;
         v[k] = x;
-    }
+    });
+    return !vanished;
 }
 
-// VA(iter) = y; M(j, iter) = <V(j), y> for j <= iter
-__global__ void __launch_bounds__(JT) jd_mcol(JdArgs a) {
-    JdState* st = a.st;
-    const int it = st->iter;
-    const double* y = Yv(a);
-    double* va = VA(a, it);
-    for (uint64_t k = lo(a) + threadIdx.x; k < hi(a); k += JT) va[k] = y[k];
-    for (int j = 0; j <= it; ++j) {
-        double p = slice_dot(a, V(a, j), y);
-        if (threadIdx.x == 0) a.partial[uint64_t(j) * gridDim.x + blockIdx.x] = p;
-    }
-    if (arrive(st)) {
-        for (int j = 0; j <= it; ++j) {
-            const double g = gather(a, j);
-            if (threadIdx.x == 0) st->M[j + it * MAXK] = g;
-        }
-        finish(a);
-    }
-}
-
-// smallest eigenpair of the leading k x k block of M (cyclic Jacobi, one warp;
-// lane r owns row/column r of the rotation updates)
-__global__ void __launch_bounds__(32) jd_ritz(JdArgs a) {
-    __shared__ double A[MAXK][MAXK + 1];
-    __shared__ double Vm[MAXK][MAXK + 1];
-    JdState* st = a.st;
-    const int k = st->iter + 1, r = threadIdx.x;
-    for (int j = 0; j < k; ++j)
-        if (r < k) {
-            A[r][j] = r <= j ? st->M[r + j * MAXK] : st->M[j + r * MAXK];
-            Vm[r][j] = r == j ? 1.0 : 0.0;
-        }
+// Smallest eigenpair of the leading k x k block of M by cyclic Jacobi, one warp, from the
+// upper triangle in sh.A (filled symmetric); theta and the vector into sh.  The rotations
+// of a sweep are the row-cyclic ones, (0,1), (0,2) .. (0,k-1), (1,2) .., taken in
+// wavefronts p + q = const: those of one wavefront touch different rows and columns and
+// every other pair of rotations keeps its order, so 2k - 3 wavefronts do what k (k - 1) / 2
+// rotations in sequence did (each a chain of a square root, a division and a reciprocal
+// square root).
+__device__ void ritz(StepShared& sh, int k) {
+    const int lane = threadIdx.x & 31;
+    for (int e = lane; e < k * k; e += 32) sh.Z[e / k][e % k] = e / k == e % k ? 1.0 : 0.0;
     __syncwarp();
     for (int sweep = 0; sweep < 100; ++sweep) {
         double off = 0.0, tot = 0.0;
-        if (r < k)
+        if (lane < k)
             for (int j = 0; j < k; ++j) {
-                double v = A[r][j] * A[r][j];
+                const double v = sh.A[lane][j] * sh.A[lane][j];
                 tot += v;
-                if (j != r) off += v;
+                if (j != lane) off += v;
             }
 #pragma unroll
         for (int o = 16; o > 0; o >>= 1) {
             off += __shfl_xor_sync(0xffffffffu, off, o);
             tot += __shfl_xor_sync(0xffffffffu, tot, o);
         }
-        off = __shfl_sync(0xffffffffu, off, 0);  // one decision for the whole warp
-        tot = __shfl_sync(0xffffffffu, tot, 0);
         if (off <= 1e-34 * tot || off == 0.0) break;
-        for (int p = 0; p < k; ++p)
-            for (int q = p + 1; q < k; ++q) {
-                const double apq = A[p][q];
-                if (apq == 0.0) continue;
-                const double app = A[p][p], aqq = A[q][q];
-                // negligible against both diagonal entries: drop it (as in jd.cu)
-                if (fabs(app) + 100.0 * fabs(apq) == fabs(app) && fabs(aqq) + 100.0 * fabs(apq) == fabs(aqq)) {
-                    __syncwarp();
-                    if (r == 0) A[p][q] = A[q][p] = 0.0;
-                    __syncwarp();
-                    continue;
+        for (int sum = 1; sum <= 2 * k - 3; ++sum) {
+            // pairs (p, sum - p), p0 <= p < (sum + 1) / 2
+            const int p0 = sum > k - 1 ? sum - (k - 1) : 0, np = (sum + 1) / 2 - p0;
+            bool any = false;
+            if (lane < np) {
+                const int p = p0 + lane, q = sum - p;
+                const double apq = sh.A[p][q], app = sh.A[p][p], aqq = sh.A[q][q];
+                double c = 1.0, s = 0.0;
+                // negligible against both diagonal entries: dropped
+                const bool drop = fabs(app) + 100.0 * fabs(apq) == fabs(app) && fabs(aqq) + 100.0 * fabs(apq) == fabs(aqq);
+                if (drop) {
+                    sh.A[p][q] = sh.A[q][p] = 0.0;
+                } else if (apq != 0.0) {
+                    const double d = aqq - app, h = 2.0 * apq;
+                    const double t = d == 0.0 ? 1.0 : h / (d + copysign(sqrt(fma(d, d, h * h)), d));
+                    const double w = fma(t, t, 1.0), c0 = rsqrt(w);
+                    c = fma(0.5 * c0, fma(-(w * c0), c0, 1.0), c0);  // to rounding
+                    s = t * c;
+                    any = true;
                 }
-                const double tau = (aqq - app) / (2.0 * apq);
-                const double tt = (tau >= 0 ? 1.0 : -1.0) / (fabs(tau) + sqrt(1.0 + tau * tau));
-                const double c = 1.0 / sqrt(1.0 + tt * tt), sn = tt * c;
-                __syncwarp();
-                if (r < k) {  // A <- A J
-                    double arp = A[r][p], arq = A[r][q];
-                    A[r][p] = c * arp - sn * arq;
-                    A[r][q] = sn * arp + c * arq;
-                }
-                __syncwarp();
-                if (r < k) {  // A <- J^T A
-                    double apr = A[p][r], aqr = A[q][r];
-                    A[p][r] = c * apr - sn * aqr;
-                    A[q][r] = sn * apr + c * aqr;
-                }
-                if (r < k) {
-                    double vrp = Vm[r][p], vrq = Vm[r][q];
-                    Vm[r][p] = c * vrp - sn * vrq;
-                    Vm[r][q] = sn * vrp + c * vrq;
-                }
-                __syncwarp();
+                sh.cs[lane][0] = c;
+                sh.cs[lane][1] = s;
             }
+            if (!__any_sync(0xffffffffu, any)) continue;
+            __syncwarp();
+            // A <- A J and Z <- Z J, then A <- J^T A
+            for (int e = lane; e < np * k; e += 32) {
+                const int r = e % k, x = e / k, p = p0 + x, q = sum - p;
+                const double c = sh.cs[x][0], s = sh.cs[x][1];
+                const double ap = sh.A[r][p], aq = sh.A[r][q], zp = sh.Z[r][p], zq = sh.Z[r][q];
+                sh.A[r][p] = c * ap - s * aq;
+                sh.A[r][q] = s * ap + c * aq;
+                sh.Z[r][p] = c * zp - s * zq;
+                sh.Z[r][q] = s * zp + c * zq;
+            }
+            __syncwarp();
+            for (int e = lane; e < np * k; e += 32) {
+                const int r = e % k, x = e / k, p = p0 + x, q = sum - p;
+                const double c = sh.cs[x][0], s = sh.cs[x][1];
+                const double ap = sh.A[p][r], aq = sh.A[q][r];
+                sh.A[p][r] = c * ap - s * aq;
+                sh.A[q][r] = s * ap + c * aq;
+            }
+            __syncwarp();
+        }
     }
     __syncwarp();
     int best = 0;
     for (int i = 1; i < k; ++i)
-        if (A[i][i] < A[best][best]) best = i;
-    if (r == 0) st->theta = A[best][best];
-    if (r < k) st->s[r] = Vm[r][best];
+        if (sh.A[i][i] < sh.A[best][best]) best = i;
+    if (lane == 0) sh.theta = sh.A[best][best];
+    if (lane < k) sh.s[lane] = sh.Z[lane][best];
 }
 
-// u = sum_j s_j V(j), uA = sum_j s_j VA(j)
-__global__ void __launch_bounds__(JT) jd_lincomb(JdArgs a) {
+// Orthogonal vectors among themselves (ietl_jacobi_davidson.h:44-48), projection of the
+// start vector (t holds x0), first basis vector.
+template <bool REG>
+__global__ void __launch_bounds__(JT) jd_start(JdArgs a) {
+    __shared__ StepShared sh;
+    unsigned phase = 0;
     JdState* st = a.st;
-    const int k = st->iter + 1;
-    double* u = U(a);
-    double* ua = UA(a);
-    for (uint64_t i = lo(a) + threadIdx.x; i < hi(a); i += JT) {
-        double x = V(a, 0)[i] * st->s[0], y = VA(a, 0)[i] * st->s[0];
+    for (int i = 0; i < a.n_ortho; ++i) {
+        Own<false> o;
+        o.g = Ov(a, i);
+        if (i > 0 && !project<false>(a, sh, phase, o, i)) return;
+        double p = 0.0;
+        each<false>(a, [&](int e, uint64_t k) { p += o.get(e, k) * o.get(e, k); });
+        if (!grid_sums(a, sh, 1, phase, [&](int, double* v) { v[0] = p; })) return;
+        // every CTA writes the same value before it reads it in project
+        if (threadIdx.x == 0) st->oo[i] = sh.sum[0];
+        __syncthreads();
+    }
+    Own<REG> t;
+    t.g = Tv(a);
+    each<REG>(a, [&](int e, uint64_t k) { t.set(e, k, Tv(a)[k]); });
+    if (a.n_ortho > 0 && !project<REG>(a, sh, phase, t, a.n_ortho)) return;
+    const bool ok = basis_vector<REG>(a, sh, phase, t, 0);
+    if (!ok && blockIdx.x == 0 && threadIdx.x == 0) cudaGraphSetConditional(a.cond, 0u);
+}
+
+// The part of an iteration after its H psi (y): projected matrix, Ritz pair, residual and
+// convergence, and, for the next iteration, the correction and the next basis vector.
+template <bool REG>
+__global__ void __launch_bounds__(JT) jd_step(JdArgs a) {
+    __shared__ StepShared sh;
+    JdState* st = a.st;
+    const int it = st->iter, k = it + 1;
+    const bool lead = blockIdx.x == 0 && threadIdx.x == 0;
+    if (lead) cudaGraphSetConditional(a.cond, 0u);
+    if (st->status) return;
+    unsigned phase = 0;
+    // VA(it) = y; M(j, it) = <V(j), y>, j <= it
+    Own<REG> y;
+    y.g = VA(a, it);
+    each<REG>(a, [&](int e, uint64_t i) {
+        const double x = Yv(a)[i];
+        y.set(e, i, x);
+        if (REG) VA(a, it)[i] = x;
+    });
+    if (!grid_sums(a, sh, k, phase, [&](int j, double* p) {
+            const double *v0 = V(a, j), *v1 = V(a, min(j + 1, it)), *v2 = V(a, min(j + 2, it)), *v3 = V(a, min(j + 3, it));
+            each<REG>(a, [&](int e, uint64_t i) {
+                const double x = y.get(e, i);
+                p[0] += v0[i] * x;
+                p[1] += v1[i] * x;
+                p[2] += v2[i] * x;
+                p[3] += v3[i] * x;
+            });
+        }))
+        return;
+    if (blockIdx.x == 0 && int(threadIdx.x) < k) st->M[threadIdx.x + it * MAXK] = sh.sum[threadIdx.x];
+    if (threadIdx.x < 32) {
+        for (int e = threadIdx.x; e < k * k; e += 32) {
+            const int r = e % k, c = e / k, lo = r < c ? r : c, hi = r < c ? c : r;
+            sh.A[r][c] = hi == it ? sh.sum[lo] : __ldcg(&st->M[lo + hi * MAXK]);
+        }
+        __syncwarp();
+        ritz(sh, k);
+    }
+    __syncthreads();
+    const double theta = sh.theta;
+    // u = sum_j s_j V(j), uA = sum_j s_j VA(j)
+    Own<REG> u, ua;
+    u.g = U(a);
+    ua.g = UA(a);
+    each<REG>(a, [&](int e, uint64_t i) {
+        double x = V(a, 0)[i] * sh.s[0], z = VA(a, 0)[i] * sh.s[0];
+#pragma unroll 4
         for (int j = 1; j < k; ++j) {
-            x += V(a, j)[i] * st->s[j];
-            y += VA(a, j)[i] * st->s[j];
+            x += V(a, j)[i] * sh.s[j];
+            z += VA(a, j)[i] * sh.s[j];
         }
-        u[i] = x;
-        ua[i] = y;
-    }
-}
-
-// r = uA - theta u; convergence test; next iteration or stop
-__global__ void __launch_bounds__(JT) jd_residual(JdArgs a) {
-    JdState* st = a.st;
-    const double theta = st->theta;
-    double* ua = UA(a);
-    const double* u = U(a);
+        u.set(e, i, x);
+        ua.set(e, i, z);
+    });
+    if (a.n_ortho > 0 && !project<REG>(a, sh, phase, ua, a.n_ortho)) return;
+    // r = uA - theta u
     double rr = 0.0, ru = 0.0, uu = 0.0;
-    for (uint64_t i = lo(a) + threadIdx.x; i < hi(a); i += JT) {
-        double r = ua[i] - theta * u[i];
-        ua[i] = r;
+    each<REG>(a, [&](int e, uint64_t i) {
+        const double x = u.get(e, i), r = ua.get(e, i) - theta * x;
+        ua.set(e, i, r);
         rr += r * r;
-        ru += r * u[i];
-        uu += u[i] * u[i];
+        ru += r * x;
+        uu += x * x;
+    });
+    if (!grid_sums(a, sh, 3, phase, [&](int, double* v) {
+            v[0] = rr;
+            v[1] = ru;
+            v[2] = uu;
+        })) return;
+    const double rnorm = sqrt(sh.sum[0]), corr = sh.sum[1] / sh.sum[2];
+    const bool conv = rnorm <= a.tol * fabs(theta) || rnorm < a.tol, done = conv || it + 1 >= a.max_iter;
+    // every CTA is past the barrier above, so none still reads st->iter
+    if (lead) {
+        st->theta = theta;
+        st->rnorm = rnorm;
+        st->iter = it + 1;
+        st->converged = conv ? 1 : 0;
+        if (done) st->done = 1;
     }
-    rr = block_sum(rr);
-    ru = block_sum(ru);
-    uu = block_sum(uu);
-    if (threadIdx.x == 0) {
-        a.partial[blockIdx.x] = rr;
-        a.partial[gridDim.x + blockIdx.x] = ru;
-        a.partial[2 * gridDim.x + blockIdx.x] = uu;
+    if (done) {
+        if (REG) each<REG>(a, [&](int e, uint64_t i) { U(a)[i] = u.get(e, i); });
+        return;
     }
-    if (arrive(st)) {
-        const double rrs = gather(a, 0), rus = gather(a, 1), uus = gather(a, 2);
-        if (threadIdx.x == 0) {
-            st->rnorm = sqrt(rrs);
-            st->corr = rus / uus;
-            st->iter += 1;
-            const bool conv = st->rnorm <= a.tol * fabs(theta) || st->rnorm < a.tol;
-            st->converged = conv ? 1 : 0;
-            if (conv || st->iter >= a.max_iter) st->done = 1;
-            cudaGraphSetConditional(a.cond, st->done ? 0u : 1u);
-        }
-        finish(a);
-    }
-}
-
-// t = -r + corr u for the next iteration
-__global__ void __launch_bounds__(JT) jd_correction(JdArgs a) {
-    JdState* st = a.st;
-    if (st->done) return;
-    const double c = st->corr;
-    const double* r = UA(a);
-    const double* u = U(a);
-    double* t = Tv(a);
-    for (uint64_t i = lo(a) + threadIdx.x; i < hi(a); i += JT) t[i] = -r[i] + c * u[i];
+    // t = -r + corr u (in place of r)
+    each<REG>(a, [&](int e, uint64_t i) { ua.set(e, i, -ua.get(e, i) + corr * u.get(e, i)); });
+    if (basis_vector<REG>(a, sh, phase, ua, it + 1) && lead) cudaGraphSetConditional(a.cond, 1u);
 }
 
 }  // namespace
@@ -435,15 +468,28 @@ void jd_graph_free(void* g) { delete static_cast<JdGraph*>(g); }
 
 namespace {
 
+cudaError_t launch_cooperative(void (*kernel)(JdArgs), int grid, JdArgs const& a, cudaStream_t s) {
+    cudaLaunchConfig_t cfg{};
+    cfg.gridDim = dim3(unsigned(grid));
+    cfg.blockDim = dim3(JT);
+    cfg.stream = s;
+    cudaLaunchAttribute attr[1];
+    attr[0].id = cudaLaunchAttributeCooperative;
+    attr[0].val.cooperative = 1;
+    cfg.attrs = attr;
+    cfg.numAttrs = 1;
+    return cudaLaunchKernelEx(&cfg, kernel, a);
+}
+
 cudaError_t build_graph(JdGraph& g, dmrgb200_plan_t plan, cudaStream_t s) {
     // s: a private non-blocking stream (the legacy default stream cannot capture)
     cudaError_t e;
     const uint64_t n = g.n;
     const int nslots = int(2 * g.max_iter + 4 + g.n_ortho);
-    const int nb = 2 * device_sm_count();
+    const int nb = device_sm_count();  // one CTA per SM: all resident, as a cooperative launch needs
     if ((e = cudaMalloc(&g.vec, sizeof(double) * n * nslots)) != cudaSuccess) return e;
     if ((e = cudaMalloc(&g.st, sizeof(JdState))) != cudaSuccess) return e;
-    if ((e = cudaMalloc(&g.partial, sizeof(double) * nb * (MAXK + 2))) != cudaSuccess) return e;
+    if ((e = cudaMalloc(&g.partial, sizeof(double) * 2 * nb * MAXK)) != cudaSuccess) return e;
     // H psi writes only block elements: the padding of every slot stays zero
     if ((e = cudaMemset(g.vec, 0, sizeof(double) * n * nslots)) != cudaSuccess) return e;
     if ((e = cudaMemset(g.st, 0, sizeof(JdState))) != cudaSuccess) return e;
@@ -453,7 +499,6 @@ cudaError_t build_graph(JdGraph& g, dmrgb200_plan_t plan, cudaStream_t s) {
     JdArgs a{};
     a.vec = g.vec;
     a.n = n;
-    a.chunk = (n + nb - 1) / nb;
     a.max_iter = int(g.max_iter);
     a.n_ortho = int(g.n_ortho);
     a.tol = g.tol;
@@ -473,24 +518,15 @@ cudaError_t build_graph(JdGraph& g, dmrgb200_plan_t plan, cudaStream_t s) {
     if ((e = cudaStreamBeginCaptureToGraph(s, g.graph, nullptr, nullptr, 0, cudaStreamCaptureModeRelaxed)) !=
         cudaSuccess)
         return e;
-    jd_init<<<1, 32, 0, s>>>(a);
-    const int no = int(g.n_ortho);
-    for (int i = 0; i < no; ++i) {
-        if (i > 0) {
-            for (int b = 0; b < i; ++b) jd_proj<<<nb, JT, 0, s>>>(a, b, 2 + i);
-            jd_proj_close<<<nb, JT, 0, s>>>(a, i - 1, 2 + i);
-        }
-        jd_oo<<<nb, JT, 0, s>>>(a, i);
-    }
-    if (no > 0) {
-        for (int i = 0; i < no; ++i) jd_proj<<<nb, JT, 0, s>>>(a, i, 0);
-        jd_proj_close<<<nb, JT, 0, s>>>(a, no - 1, 0);
-    }
+    // vectors of up to EPT elements per thread stay in registers between the passes
+    const bool reg = n <= uint64_t(EPT) * JT * nb;
+    if ((e = cudaMemsetAsync(g.st, 0, sizeof(JdState), s)) == cudaSuccess)
+        e = launch_cooperative(reg ? jd_start<true> : jd_start<false>, nb, a, s);
     cudaGraph_t captured = nullptr;
+    const cudaError_t le = e;
     e = cudaStreamEndCapture(s, &captured);
     if (e != cudaSuccess) return e;
-    e = cudaGetLastError();
-    if (e != cudaSuccess) return e;
+    if (le != cudaSuccess) return le;
 
     // the WHILE node after the prologue
     std::vector<cudaGraphNode_t> leaves;
@@ -516,32 +552,12 @@ cudaError_t build_graph(JdGraph& g, dmrgb200_plan_t plan, cudaStream_t s) {
     if ((e = cudaStreamBeginCaptureToGraph(s, body, nullptr, nullptr, 0, cudaStreamCaptureModeRelaxed)) !=
         cudaSuccess)
         return e;
-    jd_tau<<<nb, JT, 0, s>>>(a);
-    for (int pass = 0; pass < 2; ++pass) {
-        for (int j = 0; j + 1 < int(g.max_iter); ++j) jd_mgs<<<nb, JT, 0, s>>>(a, j, pass);
-        jd_mgs_close<<<nb, JT, 0, s>>>(a, pass);
-    }
-    if (no > 0) {
-        for (int i = 0; i < no; ++i) jd_proj<<<nb, JT, 0, s>>>(a, i, 0);
-        jd_proj_close<<<nb, JT, 0, s>>>(a, no - 1, 0);
-    }
-    jd_tnorm<<<nb, JT, 0, s>>>(a);
-    jd_store<<<nb, JT, 0, s>>>(a);
     cudaError_t he = plan_hpsi_launch(plan, g.vec + n * (2 * g.max_iter + 2), g.vec + n * (2 * g.max_iter + 3), s);
-    jd_mcol<<<nb, JT, 0, s>>>(a);
-    jd_ritz<<<1, 32, 0, s>>>(a);
-    jd_lincomb<<<nb, JT, 0, s>>>(a);
-    if (no > 0) {
-        for (int i = 0; i < no; ++i) jd_proj<<<nb, JT, 0, s>>>(a, i, 1);
-        jd_proj_close<<<nb, JT, 0, s>>>(a, no - 1, 1);
-    }
-    jd_residual<<<nb, JT, 0, s>>>(a);
-    jd_correction<<<nb, JT, 0, s>>>(a);
+    if (he == cudaSuccess) he = launch_cooperative(reg ? jd_step<true> : jd_step<false>, nb, a, s);
     cudaGraph_t body_out = nullptr;
     e = cudaStreamEndCapture(s, &body_out);
     if (e != cudaSuccess) return e;
     if (he != cudaSuccess) return he;
-    if ((e = cudaGetLastError()) != cudaSuccess) return e;
     return cudaGraphInstantiate(&g.exec, g.graph, 0);
 }
 
@@ -575,6 +591,9 @@ dmrgb200_status solve_graph(dmrgb200_plan_t plan, void** cache, uint64_t n, cons
         if (e != cudaSuccess) {
             delete g;
             cudaGetLastError();
+            // no cooperative kernels in graphs (a device under MPS): the caller steps on the host
+            if (e == cudaErrorNotSupported || e == cudaErrorCooperativeLaunchTooLarge)
+                return noalloc_fail(DMRGB200_NOT_SUPPORTED, "solver graph: no cooperative launch");
             return noalloc_fail(e == cudaErrorMemoryAllocation ? DMRGB200_OUT_OF_MEMORY : DMRGB200_DEVICE_ERROR,
                                 std::string("solver graph: ") + cudaGetErrorString(e));
         }
@@ -601,6 +620,7 @@ dmrgb200_status solve_graph(dmrgb200_plan_t plan, void** cache, uint64_t n, cons
 #undef CK
     float ms = 0.f;
     cudaEventElapsedTime(&ms, g->e0, g->e1);
+    if (hs.status == 2) return noalloc_fail(DMRGB200_TIMEOUT, "solver: the wait at a grid barrier ran out");
     if (hs.status) return noalloc_fail(DMRGB200_NUMERIC, "Davidson direction vanished");
     *energy = hs.theta;
     if (stats) {
