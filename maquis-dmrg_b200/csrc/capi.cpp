@@ -318,7 +318,7 @@ dmrgb200_status run_step(dmrgb200_plan_s* p, const double* ket, const double* br
             const char* v = std::getenv("DMRGB200_AUTOTUNE");
             return !(v && v[0] == '0');
         }();
-        if (tune && p->flat.flops() >= 50000000ull && !capturing(stream)) {
+        if (tune && !p->step_prog.chained && p->flat.flops() >= 50000000ull && !capturing(stream)) {
             // the variants run the whole step (outputs included): the run below rewrites them
             if ((e = tune_program(p->step_prog, reinterpret_cast<uint64_t>(ket), reinterpret_cast<uint64_t>(bra),
                                   p->step_T, p->step_S, stream)) != cudaSuccess) {
@@ -478,7 +478,8 @@ cudaError_t plan_ensure_tuned(dmrgb200_plan_t plan, const double* x, double* y, 
             e = emu_launch(plan, x, y, stream);
         return e;
     }
-    if (plan->prog.tuned) return cudaSuccess;
+    // chained products have no GEMM stages to tune
+    if (plan->prog.tuned || plan->prog.chained) return cudaSuccess;
     static const bool enabled = [] {
         const char* v = std::getenv("DMRGB200_AUTOTUNE");
         return !(v && v[0] == '0');
@@ -683,10 +684,17 @@ dmrgb200_status dmrgb200_hpsi_host(dmrgb200_plan_t plan, const double* x_host, d
     if (plan->flat.kind != KIND_HPSI || !plan->compiled) return fail(DMRGB200_INVALID_PLAN, "plan is not an H psi plan");
     cudaStream_t st = static_cast<cudaStream_t>(cuda_stream);
     cudaError_t e;
+    if (plan->pipe_built && plan->pipe.chained != plan->prog.chained) {
+        // pinned GEMM variants replaced the chained products: the ranges are lowered again
+        free_pipeline(plan->pipe);
+        if ((e = compile_pipeline(plan->flat, plan->stage3_bnd, plan->stage1_bnd, plan->prog, plan->PIPE_PARTS,
+                                  plan->pipe)) != cudaSuccess)
+            return cuda_fail(e, "host-buffer program");
+    }
     if (!plan->pipe_built) {
         plan->pipe_built = true;  // released by dmrgb200_plan_destroy, also after a failure here
-        if ((e = compile_pipeline(plan->flat, plan->stage3_bnd, plan->stage1_bnd, plan->PIPE_PARTS, plan->pipe)) !=
-            cudaSuccess)
+        if ((e = compile_pipeline(plan->flat, plan->stage3_bnd, plan->stage1_bnd, plan->prog, plan->PIPE_PARTS,
+                                  plan->pipe)) != cudaSuccess)
             return cuda_fail(e, "host-buffer program");
         const size_t nx = std::max<uint64_t>(plan->flat.in_size, 1), ny = std::max<uint64_t>(plan->flat.out_size, 1);
         if ((e = cudaMalloc(&plan->hx, nx * sizeof(double))) != cudaSuccess ||
@@ -797,6 +805,7 @@ dmrgb200_status dmrgb200_plan_set_gemm_variants(dmrgb200_plan_t plan, int32_t st
     plan->prog.var1 = stage1;
     plan->prog.var3 = stage3;
     plan->prog.tuned = true;
+    plan->prog.chained = false;  // the pinned variants are what runs
     drop_variant_graphs(plan);
     return DMRGB200_OK;
 }

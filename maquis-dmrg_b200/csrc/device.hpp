@@ -133,8 +133,60 @@ struct TileLists {
     uint32_t n[N_TILE_CLASSES] = {};
 };
 
+// a tile list on the device
+struct GemmDev {
+    DevProb* p = nullptr;
+    DevSeg* s = nullptr;
+    DevTile* t = nullptr;
+    uint32_t n = 0;
+    TileLists x;  // tile lists of the other classes
+    DevRow* r = nullptr;  // row table
+    int var = 0;  // grouped-GEMM variant
+};
+
+// ---- chained products (chain.cu): H psi and steps of plans with few terms per line ----
+// operand references: buffer id in the top 8 bits, element offset below
+struct alignas(16) DevChainTerm {
+    double alpha;
+    uint64_t p, q;  // P(k1, k2) at p + k1 p1 + k2 p2, Q(k2, n) at q + k2 q2 + n qn
+    uint64_t a;     // of the term's line: A(m, k1) at a + m am + k1 ak
+    uint32_t p1, p2, q2, qn, am, ak, k1, k2;
+    uint32_t last, pad[3];  // last term of its line
+};
+struct DevChainTile {
+    uint64_t c;              // C(m, n) at c + m cm + n cn; this tile: columns from n0
+    uint32_t n0, rows, cols, cm, cn;
+    uint32_t bounds[5];      // the tile's records in four shares of whole lines
+};
+struct ChainShape {
+    int blocks = 4;  // blocks of eight in K1 and rows a warp holds (2 to 4)
+    int split = 1;   // warps per tile
+};
+struct ChainList : ChainShape {
+    std::vector<DevChainTile> tiles;
+    std::vector<DevChainTerm> terms;
+    std::vector<uint64_t> block_off;  // per tile: offset of its H psi output block
+};
+struct ChainDev : ChainShape {
+    DevChainTile* tiles = nullptr;
+    DevChainTerm* terms = nullptr;
+    uint32_t n = 0;
+};
+// The plan as chained products, or false where it has another form (lines of many terms,
+// units that do not tile S, terms that are not whole T blocks) or larger blocks or more work
+// than the chain is faster for.
+bool build_chain(FlatPlan const& p, std::vector<uint64_t> const& stage3_bnd, std::vector<uint64_t> const& stage1_bnd,
+                 std::vector<uint64_t> const& outptr, ChainList& cl);
+cudaError_t launch_chain(ChainDev const& d, Bases const& bs, cudaStream_t stream);
+
 struct DeviceProgram {
     GemmList stage1, stage3;
+    // the whole plan as chained products (chained): what the native FP64 H psi and the boundary
+    // steps run then; the stages stay for the callers that need T or S (emulated and per-block
+    // H psi, adjoint, alpha_dm) and for pinned GEMM variants
+    bool chained = false;
+    ChainList chain;
+    ChainDev d_chain;
     std::vector<DevSLine> lines;
     std::vector<DevSTerm> terms;
     // units whose lines share sources run as line groups (see DevSGroup)
@@ -216,15 +268,6 @@ void gemm_sort_tiles(GemmList& gl);
 std::vector<uint64_t> t_offsets(FlatPlan const& p, uint64_t* total);
 std::vector<uint64_t> s_offsets(FlatPlan const& p, uint64_t* total);
 
-struct GemmDev {
-    DevProb* p = nullptr;
-    DevSeg* s = nullptr;
-    DevTile* t = nullptr;
-    uint32_t n = 0;
-    TileLists x;  // tile lists of the other classes
-    DevRow* r = nullptr;  // row table
-    int var = 0;  // grouped-GEMM variant
-};
 // grouped-GEMM variants (tile shape x pipeline depth x CTAs per SM); all sum in the
 // same order, so the choice never changes a result bit
 constexpr int N_GEMM_VARIANTS = 16;
@@ -247,9 +290,13 @@ struct PipelineProgram {
     uint32_t nparts = 0;
     std::vector<uint64_t> in_cut, out_cut;  // nparts + 1 element offsets each
     std::vector<GemmDev> s1, s3;            // device tile lists per range
+    // chained plans: the tiles of each output range (the records are the program's)
+    bool chained = false;
+    std::vector<ChainDev> ch;
 };
 cudaError_t compile_pipeline(FlatPlan const& p, std::vector<uint64_t> const& stage3_bnd,
-                             std::vector<uint64_t> const& stage1_bnd, uint32_t nparts, PipelineProgram& pp);
+                             std::vector<uint64_t> const& stage1_bnd, DeviceProgram const& prog, uint32_t nparts,
+                             PipelineProgram& pp);
 void free_pipeline(PipelineProgram& pp);
 // ev: 2 * nparts + 2 events; c: a second stream for the copies
 cudaError_t run_pipeline(DeviceProgram const& prog, PipelineProgram const& pp, const double* x_host, double* y_host,

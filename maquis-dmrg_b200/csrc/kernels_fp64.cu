@@ -1045,6 +1045,11 @@ void compile_program(FlatPlan const& p, std::vector<uint64_t> const& stage3_bnd,
         }
     }
     sort_tiles(g3);
+
+    // ---- the whole plan as chained products (the general entry points; not where an S-build form
+    // is forced) ----
+    if (stack_rows && group_lines && mode == 0 && ug_units.empty())
+        prog.chained = build_chain(p, stage3_bnd, stage1_bnd, outptr, prog.chain);
 }
 
 namespace {
@@ -1095,6 +1100,7 @@ cudaError_t upload_program(DeviceProgram& prog) {
         o_x3[c] = pk.add(prog.stage3.tiles_cls[c]);
     }
     const size_t o_l = pk.add(prog.lines), o_k = pk.add(prog.terms), o_li = pk.add(prog.litems);
+    const size_t o_ct = pk.add(prog.chain.tiles), o_cs = pk.add(prog.chain.terms);
     const size_t o_g = pk.add(prog.groups), o_gt = pk.add(prog.gent_t), o_ga = pk.add(prog.gent_a);
     const size_t o_gi = pk.add(prog.gitems);
     const size_t o_err = prog.gitems.empty() ? TablePacker::NONE : pk.zeros(sizeof(int));
@@ -1119,6 +1125,10 @@ cudaError_t upload_program(DeviceProgram& prog) {
         prog.x1.n[c] = uint32_t(prog.stage1.tiles_cls[c].size());
         prog.x3.n[c] = uint32_t(prog.stage3.tiles_cls[c].size());
     }
+    static_cast<ChainShape&>(prog.d_chain) = prog.chain;
+    prog.d_chain.tiles = at<DevChainTile>(b, o_ct);
+    prog.d_chain.terms = at<DevChainTerm>(b, o_cs);
+    prog.d_chain.n = uint32_t(prog.chain.tiles.size());
     prog.d_lines = at<DevSLine>(b, o_l);
     prog.d_terms = at<DevSTerm>(b, o_k);
     prog.d_litems = at<DevSItem>(b, o_li);
@@ -1145,6 +1155,7 @@ void free_program(DeviceProgram& prog) {
     prog.d_s3 = nullptr;
     prog.d_t3 = nullptr;
     prog.d_r1 = nullptr;
+    prog.d_chain = ChainDev();
     prog.x1 = TileLists();
     prog.x3 = TileLists();
     prog.d_lines = nullptr;
@@ -1175,12 +1186,28 @@ std::vector<uint64_t> cut_ranges(std::vector<uint64_t> const& block_off, uint64_
 }  // namespace
 
 cudaError_t compile_pipeline(FlatPlan const& p, std::vector<uint64_t> const& stage3_bnd,
-                             std::vector<uint64_t> const& stage1_bnd, uint32_t nparts, PipelineProgram& pp) {
+                             std::vector<uint64_t> const& stage1_bnd, DeviceProgram const& prog, uint32_t nparts,
+                             PipelineProgram& pp) {
     pp = PipelineProgram();
     pp.nparts = nparts;
     std::vector<uint64_t> in_off(p.in_off.begin(), p.in_off.end()), out_off(p.out_off.begin(), p.out_off.end());
     pp.in_cut = cut_ranges(in_off, p.in_size, nparts);
     pp.out_cut = cut_ranges(out_off, p.out_size, nparts);
+    if (prog.chained) {
+        pp.chained = true;
+        for (uint32_t q = 0; q < nparts; ++q) {
+            std::vector<DevChainTile> tiles;
+            for (size_t i = 0; i < prog.chain.tiles.size(); ++i)
+                if (prog.chain.block_off[i] >= pp.out_cut[q] && prog.chain.block_off[i] < pp.out_cut[q + 1])
+                    tiles.push_back(prog.chain.tiles[i]);
+            ChainDev d = prog.d_chain;
+            d.n = uint32_t(tiles.size());
+            const cudaError_t e = up(tiles, &d.tiles);
+            pp.ch.push_back(d);
+            if (e != cudaSuccess) return e;
+        }
+        return cudaSuccess;
+    }
     const std::vector<uint64_t> t_off = t_offsets(p, nullptr), s_off = s_offsets(p, nullptr);
     pp.s1.resize(nparts);
     pp.s3.resize(nparts);
@@ -1206,6 +1233,7 @@ cudaError_t compile_pipeline(FlatPlan const& p, std::vector<uint64_t> const& sta
 void free_pipeline(PipelineProgram& pp) {
     for (auto& g : pp.s1) free_gemm(g);
     for (auto& g : pp.s3) free_gemm(g);
+    for (auto& c : pp.ch) cudaFree(c.tiles);
     pp = PipelineProgram();
 }
 
@@ -1231,15 +1259,20 @@ cudaError_t run_pipeline(DeviceProgram const& prog, PipelineProgram const& pp, c
     }
     for (uint32_t q = 0; q < np; ++q) {
         if ((e = cudaStreamWaitEvent(s, ev[1 + q], 0)) != cudaSuccess) return e;
+        if (pp.chained) continue;  // every output range needs the whole input
         GemmDev g = pp.s1[q];
         g.var = prog.var1;
         if ((e = launch_gemm(g, bs, s)) != cudaSuccess) return e;
     }
-    if ((e = run_sbuild(prog, T, S, s)) != cudaSuccess) return e;
+    if (!pp.chained && (e = run_sbuild(prog, T, S, s)) != cudaSuccess) return e;
     for (uint32_t q = 0; q < np; ++q) {
-        GemmDev g = pp.s3[q];
-        g.var = prog.var3;
-        if ((e = launch_gemm(g, bs, s)) != cudaSuccess) return e;
+        if (pp.chained) {
+            if ((e = launch_chain(pp.ch[q], bs, s)) != cudaSuccess) return e;
+        } else {
+            GemmDev g = pp.s3[q];
+            g.var = prog.var3;
+            if ((e = launch_gemm(g, bs, s)) != cudaSuccess) return e;
+        }
         if ((e = cudaEventRecord(ev[1 + np + q], s)) != cudaSuccess) return e;
         if ((e = cudaStreamWaitEvent(c, ev[1 + np + q], 0)) != cudaSuccess) return e;
         const uint64_t n = pp.out_cut[q + 1] - pp.out_cut[q];
@@ -1508,6 +1541,14 @@ cudaError_t run_program(DeviceProgram const& prog, uint64_t in, uint64_t out, do
     bs.b[BUF_S] = reinterpret_cast<uint64_t>(S);
     bs.b[BUF_ABS] = 0;
     if (ev) cudaEventRecord(ev[0], stream);
+    if (prog.chained) {
+        // timed as the contraction (stage 2)
+        if (ev) cudaEventRecord(ev[1], stream);
+        if (ev) cudaEventRecord(ev[2], stream);
+        const cudaError_t e = launch_chain(prog.d_chain, bs, stream);
+        if (ev) cudaEventRecord(ev[3], stream);
+        return e != cudaSuccess ? e : cudaGetLastError();
+    }
     launch_variant(prog.var1, prog.d_p1, prog.d_s1, prog.d_t1, prog.n_t1, prog.x1, prog.d_r1, bs, stream);
     if (ev) cudaEventRecord(ev[1], stream);
     cudaError_t e = run_sbuild(prog, T, S, stream);

@@ -1,0 +1,114 @@
+"""Chained products (H·psi and boundary steps of plans with few terms per line, in one
+launch) on the device, against the oracle and against the GEMM stages (pinned variants), at sizes around the tiles: blocks of 1 to 33 rows (the chain
+takes up to 32; K1 and rows in blocks of 8, columns in tiles of 8, K2 in steps of 4)."""
+import numpy as np
+import pytest
+
+from dmrgb200 import engine as E
+from dmrgb200 import models as M
+from helpers import OracleChain, make_chain, random_psi
+
+import oracle as O
+
+torch = pytest.importorskip("torch")
+pytestmark = pytest.mark.gpu
+
+# sums of at most a few thousand FP64 products in another order: a few hundred roundings of
+# 1.1e-16, taken together in the 2-norm
+TOL = 1e-13
+
+
+def _plan(ctx, ch):
+    Lb, Rb = E.to_device(ch.Lval), E.to_device(ch.Rval)
+    plan = E.DevicePlan(ctx, ch.sched.plan, left_addr=ch.Lidx.cohort_addresses(Lb.data_ptr()),
+                        other_addr=ch.Ridx.cohort_addresses(Rb.data_ptr()))
+    return plan, (Lb, Rb)
+
+
+def _rel(a, b):
+    return np.linalg.norm(a - b) / np.linalg.norm(b)
+
+
+@pytest.mark.parametrize("name,L,m,i", [("heisenberg", 12, 5, 5), ("heisenberg", 16, 64, 3), ("heisenberg", 20, 80, 9), ("heisenberg", 20, 230, 9),
+                                        ("hubbard", 8, 12, 0), ("hubbard", 12, 60, 5), ("hubbard", 14, 333, 4),
+                                        ("hubbard", 14, 600, 6), ("hubbard", 14, 660, 6), ("bose", 10, 40, 8)])
+def test_chain_matches_oracle_and_stages(name, L, m, i):
+    ctx = E.Context(0)
+    model, bonds, tensors, rng = make_chain(name, L, 0, seed=m, synthetic_m=m)
+    ch = OracleChain(model, bonds, tensors, i)
+    plan, keep = _plan(ctx, ch)
+    x = random_psi(ch.p12, ch.left, ch.right, rng).data
+    xd = E.to_device(x)
+    yd = torch.full_like(xd, np.nan)
+    ref = ch.hpsi(x)
+    mask = np.zeros(len(ref), bool)
+    p = ch.sched.plan
+    for r, c, o in zip(p["out_rows"], p["out_cols"], p["out_off"]):
+        mask[int(o):int(o) + int(r) * int(c)] = True
+    plan.hpsi(xd.data_ptr(), yd.data_ptr())
+    torch.cuda.synchronize()
+    y = yd.cpu().numpy()
+    assert np.all(np.isnan(y[~mask]))  # the padding of y is left untouched
+    assert _rel(y[mask], ref[mask]) <= TOL
+    # host buffers run the same tiles by output range
+    xh = torch.from_numpy(x.copy()).pin_memory()
+    yh = torch.zeros_like(xh).pin_memory()
+    plan.hpsi_host(xh.data_ptr(), yh.data_ptr())
+    torch.cuda.synchronize()
+    assert np.array_equal(yh.numpy()[mask], y[mask])
+    # pinned variants run the GEMM stages, with host buffers too
+    plan.set_gemm_variants(0, 0)
+    plan.hpsi(xd.data_ptr(), yd.data_ptr())
+    plan.hpsi_host(xh.data_ptr(), yh.data_ptr())
+    torch.cuda.synchronize()
+    staged = yd.cpu().numpy()
+    assert _rel(staged[mask], ref[mask]) <= TOL
+    assert np.array_equal(yh.numpy()[mask], staged[mask])
+
+
+@pytest.mark.parametrize("name,L,m", [("heisenberg", 12, 5), ("heisenberg", 16, 130), ("hubbard", 10, 40), ("hubbard", 12, 333)])
+@pytest.mark.parametrize("symmetric", [True, False])
+def test_chain_steps_match_oracle(name, L, m, symmetric):
+    """Left steps from the left end and right steps from the right end to the middle."""
+    ctx = E.Context(0)
+    model, bonds, tensors, _ = make_chain(name, L, 0, seed=3, synthetic_m=m)
+    for left in (True, False):
+        idx = E.edge_bindex(model.symm, bonds[0] if left else bonds[L])
+        val = idx.edge_values()
+        buf = E.to_device(val)
+        for p in (range(L // 2) if left else range(L - 1, L // 2, -1)):
+            W, t = M.MPOHandle(model.mpo[p], model.symm), tensors[p]
+            if left:
+                sch, nidx = E.schedule_left_step(model.phys, bonds[p], bonds[p + 1], W, idx, symmetric)
+                val = O.left_step(sch.plan, val, idx, t.data, t.left_paired(), nidx)
+                plan = E.DevicePlan(ctx, sch.plan, left_addr=idx.cohort_addresses(buf.data_ptr()))
+                ket, bra = E.to_device(t.data), E.to_device(t.left_paired())
+            else:
+                sch, nidx = E.schedule_right_step(model.phys, bonds[p], bonds[p + 1], W, idx, symmetric)
+                val = O.right_step(sch.plan, val, idx, t.data, t.data, nidx)
+                plan = E.DevicePlan(ctx, sch.plan, other_addr=idx.cohort_addresses(buf.data_ptr()))
+                ket = bra = E.to_device(t.data)
+            out = torch.zeros(max(nidx.n_elems, 1), dtype=torch.float64, device="cuda")
+            plan.step(ket.data_ptr(), bra.data_ptr(), nidx.cohort_addresses(out.data_ptr()))
+            assert _rel(out.cpu().numpy()[:len(val)], val) <= TOL
+            idx, buf = nidx, out
+
+
+def test_chain_non_finite_boundary_stays_local():
+    """An infinite boundary element reaches the outputs that read it, as in the oracle, and
+    no others."""
+    ctx = E.Context(0)
+    model, bonds, tensors, rng = make_chain("hubbard", 10, 0, seed=2, synthetic_m=50)
+    ch = OracleChain(model, bonds, tensors, 4)
+    x = random_psi(ch.p12, ch.left, ch.right, rng).data
+    ch.Lval = ch.Lval.copy()
+    ch.Lval[int(ch.Lidx.storage_off[0])] = np.inf
+    plan, keep = _plan(ctx, ch)
+    xd = E.to_device(x)
+    yd = torch.zeros_like(xd)
+    plan.hpsi(xd.data_ptr(), yd.data_ptr())
+    torch.cuda.synchronize()
+    y, ref = yd.cpu().numpy(), ch.hpsi(x)
+    fine = np.isfinite(ref)
+    assert not fine.all() and np.all(np.isfinite(y[fine]))
+    assert _rel(y[fine], ref[fine]) <= TOL
