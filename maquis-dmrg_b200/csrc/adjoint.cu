@@ -475,6 +475,7 @@ std::string compile_adjoint(FlatPlan const& p, std::vector<uint64_t> const& stag
         gemm_add_tiles(a.g1, uint32_t(a.g1.probs.size() - 1), 1);
     }
     gemm_sort_tiles(a.g1);
+    gemm_split_long(a.g1);
 
     // ---- galpha of grouped units from the groups' Gram blocks; the rest term by term ----
     std::vector<char> grouped(p.n_terms(), 0);

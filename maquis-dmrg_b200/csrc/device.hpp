@@ -35,7 +35,23 @@ struct DevProb {
     // A operand of every segment is then read through the table, not through A.off
     // and A.ld); NO_ROWS for plain problems
     uint32_t rows = NO_ROWS;
-    static constexpr uint32_t NO_ROWS = 0xFFFFFFFFu;
+    uint32_t split = NO_SPLIT;  // entry of the list's DevSplit table: a part of a K-split problem
+    static constexpr uint32_t NO_ROWS = 0xFFFFFFFFu, NO_SPLIT = 0xFFFFFFFFu;
+};
+
+// One part of a problem whose K range is cut into `parts` (each part is a DevProb of the
+// list with its own segments).  A tile of a part stores its sums as an M x N matrix at
+// ws + part * M * N; the part that finishes a tile last (ctr + tile number) adds all parts
+// in order and stores C.
+struct DevSplit {
+    uint64_t ws;
+    uint32_t parts, part, ctr, pad;
+};
+// the table of a list with its workspace and tile counters (zero between launches)
+struct SplitArgs {
+    const DevSplit* tab = nullptr;
+    double* ws = nullptr;
+    unsigned* ctr = nullptr;
 };
 
 // one row of a row-table problem: A(r, k) = base(A.buf)[a_off + k * ld] and
@@ -125,6 +141,9 @@ struct GemmList {
     std::vector<DevTile> tiles;                        // class 0
     std::vector<DevTile> tiles_cls[N_TILE_CLASSES];    // classes 1.. (entry 0 unused)
     std::vector<DevRow> rowtab;                        // rows of row-table problems
+    std::vector<DevSplit> splits;                      // parts of K-split problems
+    uint64_t split_ws = 0;                             // workspace elements of the parts
+    uint32_t split_ctrs = 0;                           // tile counters of the parts
 };
 
 // device tile lists of the classes above 0
@@ -141,6 +160,7 @@ struct GemmDev {
     uint32_t n = 0;
     TileLists x;  // tile lists of the other classes
     DevRow* r = nullptr;  // row table
+    SplitArgs split;      // lists with K-split problems
     int var = 0;  // grouped-GEMM variant
 };
 
@@ -187,6 +207,13 @@ struct DeviceProgram {
     bool chained = false;
     ChainList chain;
     ChainDev d_chain;
+    // stage 3 with long K ranges split over CTAs (own3): what the native FP64 H psi and the
+    // steps run; stage3 itself stays for the callers that need whole problems (emulated H psi)
+    bool own3 = false;
+    uint32_t split_steps = 0;  // K steps of a part
+    GemmList stage3f;
+    GemmDev f3;
+    double* d_split_ws = nullptr;
     std::vector<DevSLine> lines;
     std::vector<DevSTerm> terms;
     // units whose lines share sources run as line groups (see DevSGroup)
@@ -264,6 +291,8 @@ cudaError_t scale_buffer(double* x, uint64_t n, double a, cudaStream_t st);
 DevOp dev_op(uint16_t buf, uint64_t off, uint32_t ld, bool trans, uint64_t bstride = 0);
 void gemm_add_tiles(GemmList& gl, uint32_t prob, uint32_t nbatch);
 void gemm_sort_tiles(GemmList& gl);
+// long K ranges of a list of few tiles cut into parts
+void gemm_split_long(GemmList& gl);
 // element offsets of the plan's T matrices / S matrices in the scratch buffers
 std::vector<uint64_t> t_offsets(FlatPlan const& p, uint64_t* total);
 std::vector<uint64_t> s_offsets(FlatPlan const& p, uint64_t* total);

@@ -17,6 +17,7 @@
 #include <numeric>
 #include <tuple>
 #include <string>
+#include <type_traits>
 #include <unordered_map>
 
 #include "../../include/dmrgb200.h"
@@ -56,6 +57,10 @@ __device__ __forceinline__ void cp_async8(double* smem, const double* gmem, bool
     int n = valid ? 8 : 0;
     asm volatile("cp.async.ca.shared.global [%0], [%1], 8, %2;\n" ::"r"(saddr), "l"(gmem), "r"(n));
 }
+__device__ __forceinline__ void cp_async8_all(double* smem, const char* gmem) {
+    unsigned saddr = static_cast<unsigned>(__cvta_generic_to_shared(smem));
+    asm volatile("cp.async.ca.shared.global [%0], [%1], 8;\n" ::"r"(saddr), "l"(gmem));
+}
 __device__ __forceinline__ void cp_async_commit() { asm volatile("cp.async.commit_group;\n" ::); }
 template <int N>
 __device__ __forceinline__ void cp_async_wait() {
@@ -77,7 +82,12 @@ __device__ __forceinline__ int swz(int k) { return (k >> 2) & 3; }
 // transposed), the thread's copies share one row r = tid % ROWS and take
 // k = kt + j * (NTHREADS / ROWS); otherwise they share k = kt = tid % BK_ and
 // take rows r + j * (NTHREADS / BK_).  Copy j reads base + j * jstride; every
-// K step advances base by kstep.  All byte strides, fixed per segment.
+// K step advances base by kstep.  All byte strides, fixed per segment.  Rows outside the
+// problem are not copied: what the tile holds there only reaches outputs that are not
+// stored.  A whole K step has no per-copy conditions (about five instructions per copy
+// instead of ten: on blocks of 17 to 52 rows the copies' arithmetic is most of what the
+// kernel executes); the last one of a segment zero-fills its K rows past the end, up to the
+// DMMA step of four that is multiplied.
 struct CopyStream {
     const char* base;
     const char* safe;  // a readable address for copies that fetch nothing
@@ -92,21 +102,40 @@ __device__ __forceinline__ void issue_copies(double* tile, CopyStream& cs, uint3
     constexpr int NC = ROWS * BK_ / NTHREADS;
     if (cs.rowmajor) {
         constexpr int KJ = NTHREADS / ROWS;
+        static_assert(KJ <= 4 || NC == 1 || KJ % 4 == 0, "swizzle of copy j");
+        if (cs.mask) {
+            const char* p = cs.base;
+            // swz(kt + j KJ): kt < KJ, so for KJ <= 4 it depends on j alone
+            const uint32_t t0 = KJ <= 4 ? 0u : cs.kt >> 2;
+            if (krem >= uint32_t(BK_)) {
 #pragma unroll
-        for (int j = 0; j < NC; ++j) {
-            const uint32_t k = cs.kt + j * KJ;
-            const bool ok = ((cs.mask >> j) & 1u) && k < krem;
-            cp_async8(&tile[k * LD + (cs.r ^ swz(k))],
-                      reinterpret_cast<const double*>(ok ? cs.base + j * cs.jstride : cs.safe), ok);
+                for (int j = 0; j < NC; ++j, p += cs.jstride)
+                    cp_async8_all(&tile[(cs.kt + j * KJ) * LD + (cs.r ^ ((t0 + ((j * KJ) >> 2)) & 3u))], p);
+            } else {
+                const uint32_t kend = (krem + 3u) & ~3u;
+#pragma unroll
+                for (int j = 0; j < NC; ++j, p += cs.jstride) {
+                    const uint32_t k = cs.kt + j * KJ;
+                    if (k < kend)
+                        cp_async8(&tile[k * LD + (cs.r ^ swz(k))], reinterpret_cast<const double*>(k < krem ? p : cs.safe),
+                                  k < krem);
+                }
+            }
         }
     } else {
         constexpr int RJ = NTHREADS / BK_;
+        static_assert(RJ % 4 == 0, "swizzle of copy j");
+        double* dst = &tile[cs.kt * LD + (cs.r ^ swz(cs.kt))];  // (r + j RJ) ^ swz = (r ^ swz) + j RJ
+        const char* p = cs.base;
         const bool kok = cs.kt < krem;
+        if (krem >= uint32_t(BK_)) {
 #pragma unroll
-        for (int j = 0; j < NC; ++j) {
-            const bool ok = kok && ((cs.mask >> j) & 1u);
-            cp_async8(&tile[cs.kt * LD + ((cs.r + j * RJ) ^ swz(cs.kt))],
-                      reinterpret_cast<const double*>(ok ? cs.base + j * cs.jstride : cs.safe), ok);
+            for (int j = 0; j < NC; ++j, p += cs.jstride)
+                if ((cs.mask >> j) & 1u) cp_async8_all(dst + j * RJ, p);
+        } else if (cs.kt < ((krem + 3u) & ~3u)) {
+#pragma unroll
+            for (int j = 0; j < NC; ++j, p += cs.jstride)
+                if ((cs.mask >> j) & 1u) cp_async8(dst + j * RJ, reinterpret_cast<const double*>(kok ? p : cs.safe), kok);
         }
     }
     cs.base += cs.kstep;
@@ -158,7 +187,8 @@ template <int BM_, int BN_, int BK_, int STAGES, int MINB, int NTHREADS, int WAR
 __global__ void __launch_bounds__(NTHREADS, MINB) gemm_f64_grouped(const DevProb* __restrict__ probs,
                                                                    const DevSeg* __restrict__ segs,
                                                                    const DevTile* __restrict__ tiles, uint32_t n_tiles,
-                                                                   const DevRow* __restrict__ rowtab, Bases bases) {
+                                                                   const DevRow* __restrict__ rowtab, SplitArgs split,
+                                                                   Bases bases) {
     // warps: WARPS_M x (warps / WARPS_M), warp tiles WM x WN of 8 x 8 DMMA tiles
     constexpr int WM = BM_ / WARPS_M;
     constexpr int WN = BN_ / (NTHREADS / 32 / WARPS_M), NJ = WN / 8;
@@ -168,6 +198,8 @@ __global__ void __launch_bounds__(NTHREADS, MINB) gemm_f64_grouped(const DevProb
                   "tile shape");
     __shared__ __align__(16) double As[STAGES][BK_][pitch<BM_>()];
     __shared__ __align__(16) double Bs[STAGES][BK_][pitch<BN_>()];
+    __shared__ uint32_t st_k[STAGES];  // K rows a stage holds
+    __shared__ uint32_t st_last;       // this tile's part arrived last (K-split problems)
     wait_for_predecessor();
 
     const int tid = threadIdx.x;
@@ -225,6 +257,7 @@ __global__ void __launch_bounds__(NTHREADS, MINB) gemm_f64_grouped(const DevProb
     };
     auto issue = [&](int slot) {
         if (!L.valid) return;
+        if (tid == 0) st_k[slot] = L.seg < L.seg_end ? min(L.krem, uint32_t(BK_)) : 0u;
         if (L.seg < L.seg_end) {  // an empty tile issues no copies
             issue_copies<BM_, BK_, NTHREADS, pitch<BM_>()>(&As[slot][0][0], ca, L.krem);
             issue_copies<BN_, BK_, NTHREADS, pitch<BN_>()>(&Bs[slot][0][0], cb, L.krem);
@@ -256,34 +289,89 @@ __global__ void __launch_bounds__(NTHREADS, MINB) gemm_f64_grouped(const DevProb
     // ---- consumer: tiles in the same order, nsteps K steps each ----
     int slot = 0;
     for (uint32_t ti = blockIdx.x; ti < n_tiles; ti += gridDim.x) {
-        const uint32_t nsteps = tiles[ti].nsteps;
-        for (uint32_t st = 0; st < nsteps; ++st) {
+        const DevTile tl = tiles[ti];
+        const DevProb& pr = probs[tl.prob];
+        const uint32_t M = pr.M, N = pr.N;
+        const bool inside = tl.m0 + wm < M && tl.n0 + wn < N;  // any of this warp's tile
+        for (uint32_t st = 0; st < tl.nsteps; ++st) {
             issue((slot + STAGES - 1) % STAGES);
             cp_async_commit();
             cp_async_wait<STAGES - 1>();
             __syncthreads();
+            // K steps of four past the segment's end are not multiplied, nor tiles of warps outside
+            // the problem; the unrolled forms keep the fragment reads ahead of the products (a
+            // condition per step of four costs more than it saves: Heisenberg m = 1024 stage 3
+            // 52 us instead of 44)
+            const uint32_t kn = (st_k[slot] + 3u) / 4u;
+            if (inside) {
+                auto product = [&](auto steps) {
+                    constexpr int KS = decltype(steps)::value;
 #pragma unroll
-            for (int kk = 0; kk < BK_; kk += 4) {
-                double a[MI], b[NJ];
+                    for (int kk = 0; kk < 4 * KS; kk += 4) {
+                        double a[MI], b[NJ];
 #pragma unroll
-                for (int i = 0; i < MI; ++i) a[i] = As[slot][kk + q][(wm + i * 8 + g) ^ (kk >> 2)];
+                        for (int i = 0; i < MI; ++i) a[i] = As[slot][kk + q][(wm + i * 8 + g) ^ (kk >> 2)];
 #pragma unroll
-                for (int j = 0; j < NJ; ++j) b[j] = Bs[slot][kk + q][(wn + j * 8 + g) ^ (kk >> 2)];
+                        for (int j = 0; j < NJ; ++j) b[j] = Bs[slot][kk + q][(wn + j * 8 + g) ^ (kk >> 2)];
 #pragma unroll
-                for (int i = 0; i < MI; ++i)
+                        for (int i = 0; i < MI; ++i)
 #pragma unroll
-                    for (int j = 0; j < NJ; ++j) dmma(acc[i][j][0], acc[i][j][1], a[i], b[j]);
+                            for (int j = 0; j < NJ; ++j) dmma(acc[i][j][0], acc[i][j][1], a[i], b[j]);
+                    }
+                };
+                if (kn == BK_ / 4) product(std::integral_constant<int, BK_ / 4>());
+                else if (kn == 1) product(std::integral_constant<int, 1>());
+                else if (BK_ > 8 && kn == 2) product(std::integral_constant<int, 2>());
+                else if (BK_ > 8 && kn == 3) product(std::integral_constant<int, 3>());
             }
             __syncthreads();
             slot = (slot + 1) % STAGES;
         }
-        // epilogue (the next tile's first steps are already in flight); an empty
-        // tile's single step multiplied zero-filled or stale shared memory, so its
-        // accumulators are cleared instead of stored
-        const DevTile tl = tiles[ti];
-        const DevProb pr = probs[tl.prob];
-        bool empty = true;
-        for (uint32_t sg = pr.seg_begin; sg < pr.seg_end; ++sg) empty = empty && segs[sg].K == 0;
+        // epilogue (the next tile's first steps are already in flight); an empty tile multiplied
+        // nothing and stores zeros
+        if (pr.split != DevProb::NO_SPLIT) {
+            const DevSplit sp = split.tab[pr.split];
+            const uint64_t mn = uint64_t(M) * N;
+            double* part = split.ws + sp.ws + sp.part * mn;
+#pragma unroll
+            for (int i = 0; i < MI; ++i)
+#pragma unroll
+                for (int j = 0; j < NJ; ++j)
+#pragma unroll
+                    for (int e = 0; e < 2; ++e) {
+                        const uint32_t r = tl.m0 + wm + i * 8 + g, c = tl.n0 + wn + j * 8 + q * 2 + e;
+                        if (r < M && c < N) __stcg(part + r + uint64_t(c) * M, acc[i][j][e]);
+                    }
+            // the last part to arrive sees every part's sums (release and acquire around the count)
+            __threadfence();
+            __syncthreads();
+            if (tid == 0) {
+                unsigned* ctr = split.ctr + sp.ctr + (tl.m0 / BM_) * ((N + BN_ - 1) / BN_) + tl.n0 / BN_;
+                const bool last = atomicAdd(ctr, 1u) == sp.parts - 1;
+                if (last) *ctr = 0;
+                st_last = last ? 1u : 0u;
+                __threadfence();
+            }
+            __syncthreads();
+            const bool last = st_last != 0;
+#pragma unroll
+            for (int i = 0; i < MI; ++i)
+#pragma unroll
+                for (int j = 0; j < NJ; ++j) acc[i][j][0] = acc[i][j][1] = 0.0;
+            // part by part, all of a thread's elements of one part in flight at once
+            const double* ws = split.ws + sp.ws;
+            for (uint32_t x = 0; last && x < sp.parts; ++x, ws += mn)
+#pragma unroll
+                for (int i = 0; i < MI; ++i)
+#pragma unroll
+                    for (int j = 0; j < NJ; ++j)
+#pragma unroll
+                        for (int e = 0; e < 2; ++e) {
+                            const uint32_t r = tl.m0 + wm + i * 8 + g, c = tl.n0 + wn + j * 8 + q * 2 + e;
+                            if (r < M && c < N) acc[i][j][e] += __ldcg(ws + r + uint64_t(c) * M);
+                        }
+            if (!last) continue;
+        }
         const bool rowmode = pr.rows != DevProb::NO_ROWS;
         double* C = const_cast<double*>(op_base(bases, pr.C, tl.batch));
         const uint64_t ldc = pr.C.ld;
@@ -293,7 +381,7 @@ __global__ void __launch_bounds__(NTHREADS, MINB) gemm_f64_grouped(const DevProb
             // the row's start and leading dimension: from the row table or the plain operand
             double* crow = C + r;
             uint64_t ld = ldc;
-            if (rowmode && r < pr.M) {
+            if (rowmode && r < M) {
                 const DevRow rw = rowtab[pr.rows + r];
                 crow = reinterpret_cast<double*>(base_of(bases, pr.C.buf) + 8ull * (rw.c_off + tl.batch * rw.cbs));
                 ld = rw.ld;
@@ -303,7 +391,7 @@ __global__ void __launch_bounds__(NTHREADS, MINB) gemm_f64_grouped(const DevProb
 #pragma unroll
                 for (int e = 0; e < 2; ++e) {
                     uint32_t c = tl.n0 + wn + j * 8 + q * 2 + e;
-                    if (r < pr.M && c < pr.N) crow[c * ld] = empty ? 0.0 : acc[i][j][e];
+                    if (r < M && c < N) crow[c * ld] = acc[i][j][e];
                     acc[i][j][e] = 0.0;
                 }
         }
@@ -633,30 +721,53 @@ std::vector<uint64_t> s_offsets(FlatPlan const& p, uint64_t* total) {
 }
 
 namespace {
+// Blocks of every T task that some term reads; the others are never used (at the middle
+// of a Fermi-Hubbard chain the tasks hold 2312 blocks of which 1624 are read).
+std::vector<std::vector<char>> t_blocks_read(FlatPlan const& p) {
+    std::vector<std::vector<char>> read(p.n_t());
+    for (uint32_t t = 0; t < p.n_t(); ++t) read[t].assign(p.t_nb[t], 0);
+    for (uint32_t u = 0; u < p.n_units(); ++u)
+        for (uint32_t l = p.u_line[u]; l < p.u_line[u + 1]; ++l)
+            for (uint32_t k = p.l_term[l]; k < p.l_term[l + 1]; ++k) {
+                // columns term_col .. + u_ms of the task's T, usually one whole block
+                const uint32_t t = p.term_t[k], w = p.t_bcols[t];
+                if (!w || !p.u_ms[u]) continue;
+                for (uint32_t b = p.term_col[k] / w; b <= (p.term_col[k] + p.u_ms[u] - 1) / w && b < p.t_nb[t]; ++b)
+                    read[t][b] = 1;
+            }
+    return read;
+}
+
 // Stage 1 of H psi / right step with the rows of all T tasks that share a
 // boundary cohort (same cohort, transposition and shape) stacked into one
 // row-table problem: A row r is row r' of task t's psi slice, C row r is row r'
 // of T_t (leading dimension = the task's row count), so one tile covers several
-// small psi blocks instead of padding each to a full tile.
+// small psi blocks instead of padding each to a full tile.  T blocks that no term reads
+// are left out where that saves a tenth of a cohort's blocks or more: the tasks are then
+// stacked by the set of blocks they need, one problem per run of adjacent blocks.  (In
+// quantum chemistry nearly all blocks are read, by slightly different sets per task:
+// splitting there would undo the stacking for a percent of the work.)
 void stack_stage1(FlatPlan const& p, std::vector<uint64_t> const& stage1_bnd, std::vector<uint64_t> const& t_off,
-                  GemmList& g1, std::vector<char> const* keep = nullptr) {
+                  GemmList& g1, std::vector<char> const* keep = nullptr, bool skip_unread = false) {
     g1 = GemmList();
     std::map<std::tuple<uint32_t, uint8_t, uint32_t, uint32_t, uint32_t>, std::vector<uint32_t>> groups;
     for (uint32_t t = 0; t < p.n_t(); ++t)
         if (!keep || (*keep)[t]) groups[{p.t_ci[t], p.t_trans[t], p.t_brows[t], p.t_bcols[t], p.t_nb[t]}].push_back(t);
-    for (auto const& kv : groups) {
-        const uint32_t t0 = kv.second.front();
-        const uint32_t K = p.t_brows[t0], Nf = p.t_bcols[t0], nb = p.t_nb[t0];
+    std::vector<std::vector<char>> read;
+    if (skip_unread) read = t_blocks_read(p);
+    auto problem = [&](std::vector<uint32_t> const& tasks, uint32_t b0, uint32_t nb) {
+        const uint32_t t0 = tasks.front();
+        const uint32_t K = p.t_brows[t0], Nf = p.t_bcols[t0];
         const bool tr = p.t_trans[t0] != 0;
-        const uint64_t bnd = stage1_bnd.at(p.t_ci[t0]) / 8;
+        const uint64_t bnd = stage1_bnd.at(p.t_ci[t0]) / 8 + uint64_t(b0) * K * Nf;
         DevProb pr;
         pr.rows = uint32_t(g1.rowtab.size());
         uint32_t M = 0;
-        for (uint32_t t : kv.second) {
+        for (uint32_t t : tasks) {
             const uint32_t Mt = p.in_rows[p.t_lb[t]];
             for (uint32_t r = 0; r < Mt; ++r)
-                g1.rowtab.push_back(DevRow{p.in_off[p.t_lb[t]] + uint64_t(p.t_col[t]) * Mt + r, t_off[t] + r,
-                                           tr ? uint64_t(Mt) * Nf : 0, Mt, 0});
+                g1.rowtab.push_back(DevRow{p.in_off[p.t_lb[t]] + uint64_t(p.t_col[t]) * Mt + r,
+                                           t_off[t] + uint64_t(b0) * Mt * Nf + r, tr ? uint64_t(Mt) * Nf : 0, Mt, 0});
             M += Mt;
         }
         pr.M = M;
@@ -679,6 +790,25 @@ void stack_stage1(FlatPlan const& p, std::vector<uint64_t> const& stage1_bnd, st
         pr.seg_end = uint32_t(g1.segs.size());
         g1.probs.push_back(pr);
         add_tiles(g1, uint32_t(g1.probs.size() - 1), nbatch);
+    };
+    for (auto const& kv : groups) {
+        const uint32_t nb = p.t_nb[kv.second.front()];
+        uint64_t used = 0;
+        if (skip_unread)
+            for (uint32_t t : kv.second) used += uint64_t(std::count(read[t].begin(), read[t].end(), 1));
+        if (!skip_unread || used * 10 > uint64_t(nb) * kv.second.size() * 9) {
+            problem(kv.second, 0, nb);
+            continue;
+        }
+        std::map<std::vector<char>, std::vector<uint32_t>> by_set;
+        for (uint32_t t : kv.second) by_set[read[t]].push_back(t);
+        for (auto const& sv : by_set)
+            for (uint32_t b = 0; b < nb;) {
+                uint32_t e = b;
+                while (e < nb && sv.first[e]) ++e;
+                if (e > b) problem(sv.second, b, e - b);
+                b = e + 1;
+            }
     }
     sort_tiles(g1);
 }
@@ -840,6 +970,84 @@ void build_stage3_hpsi(FlatPlan const& p, std::vector<uint64_t> const& stage3_bn
 }
 }  // namespace
 
+namespace {
+// K steps (of 16) of a part when long problems are cut: half of what each of the CTAs that
+// fill the chip (four per SM) would get if the list's work were spread evenly, so that the
+// parts also balance.  At least 48: storing, counting and adding a tile's partial sums costs
+// a CTA about 4 us, and shorter parts lose (at the Hubbard middle of m = 1024, 6 to 24 steps per
+// tile, parts of 8 took 41 us where whole tiles take 27).  In quantum chemistry stage 3 has one
+// problem per output block: at L = 12, m = 300 10 problems of 107 to 382 steps, whose 127 tiles
+// of 16 x 64 took 220 us whole and take 104 us in parts.
+uint32_t split_target(GemmList const& gl) {
+    uint64_t total = 0;
+    for (auto const& t : gl.tiles) total += t.nsteps;
+    return uint32_t(std::max<uint64_t>(48, total / (2 * 4 * 148)));
+}
+
+// `gl` with K ranges of more than `target` steps cut into parts, a function of the problem and
+// the target alone (the sums do not depend on the list a problem stands in nor on the kernel
+// variant).  Returns false where nothing is cut: the tiles are many, or short.
+bool split_list(GemmList const& gl, uint32_t target, GemmList& out) {
+    out = GemmList();
+    bool any = false;
+    std::vector<uint32_t> nbatch(gl.probs.size(), 0);
+    for (auto const& t : gl.tiles) nbatch[t.prob] = std::max(nbatch[t.prob], t.batch + 1);
+    for (uint32_t i = 0; i < gl.probs.size(); ++i) {
+        DevProb pr = gl.probs[i];
+        uint64_t steps = 0;
+        for (uint32_t s = pr.seg_begin; s < pr.seg_end; ++s) steps += (gl.segs[s].K + 15) / 16;
+        const uint32_t parts = nbatch[i] == 1 && pr.rows == DevProb::NO_ROWS && pr.M && pr.N
+                                   ? uint32_t(std::min<uint64_t>((steps + target - 1) / target, 16))
+                                   : 1;
+        uint32_t sg = pr.seg_begin, koff = 0;  // next segment and the K rows of it already given out
+        uint64_t given = 0;
+        const uint64_t ws = out.split_ws;
+        const uint32_t ctr = out.split_ctrs;
+        for (uint32_t x = 0; x < parts; ++x) {
+            DevProb q = pr;
+            q.seg_begin = uint32_t(out.segs.size());
+            // steps [given, upto) of the problem: whole segments, or pieces of 16 K rows
+            const uint64_t upto = steps * (x + 1) / parts;
+            while (sg < pr.seg_end && (given < upto || x + 1 == parts)) {
+                DevSeg piece = gl.segs[sg];
+                const uint32_t left = piece.K - koff, here = (left + 15) / 16;
+                const uint32_t take = x + 1 == parts ? left : uint32_t(std::min<uint64_t>(left, (upto - given) * 16));
+                piece.A.off += piece.A.trans ? koff : uint64_t(koff) * piece.A.ld;
+                piece.B.off += piece.B.trans ? uint64_t(koff) * piece.B.ld : koff;
+                piece.K = take;
+                if (take) out.segs.push_back(piece);
+                given += take == left ? here : (take + 15) / 16;
+                koff += take;
+                if (koff == gl.segs[sg].K) {
+                    ++sg;
+                    koff = 0;
+                }
+            }
+            q.seg_end = uint32_t(out.segs.size());
+            if (parts > 1) {
+                any = true;
+                q.split = uint32_t(out.splits.size());
+                out.splits.push_back(DevSplit{ws, parts, x, ctr, 0});
+            }
+            out.probs.push_back(q);
+            add_tiles(out, uint32_t(out.probs.size() - 1), nbatch[i]);
+        }
+        if (parts > 1) {
+            out.split_ws += uint64_t(parts) * pr.M * pr.N;
+            // counters for the smallest tiles of any class (16 rows, 32 columns)
+            out.split_ctrs += ((pr.M + 15) / 16) * ((pr.N + 31) / 32);
+        }
+    }
+    out.rowtab = gl.rowtab;
+    if (!any) {
+        out = GemmList();
+        return false;
+    }
+    sort_tiles(out);
+    return true;
+}
+}  // namespace
+
 void compile_program(FlatPlan const& p, std::vector<uint64_t> const& stage3_bnd,
                      std::vector<uint64_t> const& stage1_bnd, std::vector<uint64_t> const& outptr,
                      DeviceProgram& prog, bool stack_rows, bool group_lines) {
@@ -892,7 +1100,7 @@ void compile_program(FlatPlan const& p, std::vector<uint64_t> const& stage3_bnd,
     sort_tiles(g1);
     if (stack_rows && p.kind != KIND_LEFT && p.n_t()) {
         prog.stage1_tasks = std::move(prog.stage1);
-        stack_stage1(p, stage1_bnd, t_off, prog.stage1);
+        stack_stage1(p, stage1_bnd, t_off, prog.stage1, nullptr, group_lines);
     }
 
     // ---- stage 2 (S lines) ----
@@ -1050,6 +1258,11 @@ void compile_program(FlatPlan const& p, std::vector<uint64_t> const& stage3_bnd,
     // is forced) ----
     if (stack_rows && group_lines && mode == 0 && ug_units.empty())
         prog.chained = build_chain(p, stage3_bnd, stage1_bnd, outptr, prog.chain);
+    // ---- stage 3 with long K ranges split ----
+    if (stack_rows && group_lines && g3.tiles.size() < 4 * 4 * 148) {
+        prog.split_steps = split_target(g3);
+        prog.own3 = split_list(g3, prog.split_steps, prog.stage3f);
+    }
 }
 
 namespace {
@@ -1100,6 +1313,11 @@ cudaError_t upload_program(DeviceProgram& prog) {
         o_x3[c] = pk.add(prog.stage3.tiles_cls[c]);
     }
     const size_t o_l = pk.add(prog.lines), o_k = pk.add(prog.terms), o_li = pk.add(prog.litems);
+    const size_t o_pf = pk.add(prog.stage3f.probs), o_sf = pk.add(prog.stage3f.segs), o_tf = pk.add(prog.stage3f.tiles);
+    const size_t o_sp = pk.add(prog.stage3f.splits);
+    const size_t o_cn = prog.stage3f.split_ctrs ? pk.zeros(prog.stage3f.split_ctrs * sizeof(unsigned)) : TablePacker::NONE;
+    size_t o_xf[N_TILE_CLASSES];
+    for (int c = 1; c < N_TILE_CLASSES; ++c) o_xf[c] = pk.add(prog.stage3f.tiles_cls[c]);
     const size_t o_ct = pk.add(prog.chain.tiles), o_cs = pk.add(prog.chain.terms);
     const size_t o_g = pk.add(prog.groups), o_gt = pk.add(prog.gent_t), o_ga = pk.add(prog.gent_a);
     const size_t o_gi = pk.add(prog.gitems);
@@ -1124,6 +1342,20 @@ cudaError_t upload_program(DeviceProgram& prog) {
         prog.x3.t[c] = at<DevTile>(b, o_x3[c]);
         prog.x1.n[c] = uint32_t(prog.stage1.tiles_cls[c].size());
         prog.x3.n[c] = uint32_t(prog.stage3.tiles_cls[c].size());
+    }
+    prog.f3 = GemmDev();
+    if (prog.own3) {
+        const cudaError_t e = cudaMalloc(&prog.d_split_ws, prog.stage3f.split_ws * sizeof(double));
+        if (e != cudaSuccess) return e;
+        prog.f3.split = SplitArgs{at<DevSplit>(b, o_sp), prog.d_split_ws, at<unsigned>(b, o_cn)};
+        prog.f3.p = at<DevProb>(b, o_pf);
+        prog.f3.s = at<DevSeg>(b, o_sf);
+        prog.f3.t = at<DevTile>(b, o_tf);
+        prog.f3.n = uint32_t(prog.stage3f.tiles.size());
+        for (int c = 1; c < N_TILE_CLASSES; ++c) {
+            prog.f3.x.t[c] = at<DevTile>(b, o_xf[c]);
+            prog.f3.x.n[c] = uint32_t(prog.stage3f.tiles_cls[c].size());
+        }
     }
     static_cast<ChainShape&>(prog.d_chain) = prog.chain;
     prog.d_chain.tiles = at<DevChainTile>(b, o_ct);
@@ -1155,6 +1387,9 @@ void free_program(DeviceProgram& prog) {
     prog.d_s3 = nullptr;
     prog.d_t3 = nullptr;
     prog.d_r1 = nullptr;
+    cudaFree(prog.d_split_ws);
+    prog.d_split_ws = nullptr;
+    prog.f3 = GemmDev();
     prog.d_chain = ChainDev();
     prog.x1 = TileLists();
     prog.x3 = TileLists();
@@ -1220,9 +1455,11 @@ cudaError_t compile_pipeline(FlatPlan const& p, std::vector<uint64_t> const& sta
         for (uint32_t ob = 0; ob < p.out_rows.size(); ++ob)
             keep_o[ob] = p.out_off[ob] >= pp.out_cut[q] && p.out_off[ob] < pp.out_cut[q + 1];
         GemmList g1, g3;
-        stack_stage1(p, stage1_bnd, t_off, g1, &keep_t);
+        stack_stage1(p, stage1_bnd, t_off, g1, &keep_t, true);
         build_stage3_hpsi(p, stage3_bnd, s_off, g3, &keep_o);
         sort_tiles(g3);
+        GemmList g3s;  // the whole plan's K parts, so that the sums are the same
+        if (prog.own3 && split_list(g3, prog.split_steps, g3s)) g3 = std::move(g3s);
         cudaError_t e;
         if ((e = upload_gemm(g1, pp.s1[q])) != cudaSuccess) return e;
         if ((e = upload_gemm(g3, pp.s3[q])) != cudaSuccess) return e;
@@ -1307,6 +1544,11 @@ double calibrate_fp64_tflops() {
     return ms > 0 ? flops / (ms * 1e-3) / 1e12 : 0.0;
 }
 
+void gemm_split_long(GemmList& gl) {
+    GemmList cut;
+    if (gl.tiles.size() < 4 * 4 * 148 && split_list(gl, split_target(gl), cut)) gl = std::move(cut);
+}
+
 cudaError_t upload_gemm(GemmList const& gl, GemmDev& d) {
     cudaError_t e;
     if ((e = up(gl.probs, &d.p)) != cudaSuccess) return e;
@@ -1318,7 +1560,13 @@ cudaError_t upload_gemm(GemmList const& gl, GemmDev& d) {
         d.x.n[c] = uint32_t(gl.tiles_cls[c].size());
     }
     d.n = uint32_t(gl.tiles.size());
-
+    if (!gl.splits.empty()) {
+        DevSplit* tab = nullptr;
+        if ((e = up(gl.splits, &tab)) != cudaSuccess) return e;
+        d.split.tab = tab;
+        if ((e = cudaMalloc(&d.split.ws, gl.split_ws * sizeof(double))) != cudaSuccess) return e;
+        if ((e = up(std::vector<unsigned>(gl.split_ctrs, 0u), &d.split.ctr)) != cudaSuccess) return e;
+    }
     return cudaSuccess;
 }
 
@@ -1328,11 +1576,15 @@ void free_gemm(GemmDev& d) {
     cudaFree(d.t);
     for (int c = 1; c < N_TILE_CLASSES; ++c) cudaFree(d.x.t[c]);
     cudaFree(d.r);
+    cudaFree(const_cast<DevSplit*>(d.split.tab));
+    cudaFree(d.split.ws);
+    cudaFree(d.split.ctr);
     d = GemmDev();
 }
 
 namespace {
-using GemmKernel = void (*)(const DevProb*, const DevSeg*, const DevTile*, uint32_t, const DevRow*, Bases);
+using GemmKernel = void (*)(const DevProb*, const DevSeg*, const DevTile*, uint32_t, const DevRow*, SplitArgs,
+                            Bases);
 
 // pipeline depth x CTAs per SM of the grouped GEMM, chosen per stage by the autotuner
 struct GemmVariant {
@@ -1392,7 +1644,8 @@ cudaError_t launch_pdl(void (*kernel)(KArgs...), uint32_t grid, uint32_t block, 
 }
 
 cudaError_t launch_variant(int v, const DevProb* p, const DevSeg* sg, const DevTile* t, uint32_t n,
-                           TileLists const& x, const DevRow* rows, Bases const& bs, cudaStream_t stream) {
+                           TileLists const& x, const DevRow* rows, SplitArgs const& split, Bases const& bs,
+                           cudaStream_t stream) {
     if (!n) return cudaSuccess;
     if (v < 0 || v >= N_GEMM_VARIANTS) v = 0;
     const int c = kVariants[v].tile_class;
@@ -1402,14 +1655,14 @@ cudaError_t launch_variant(int v, const DevProb* p, const DevSeg* sg, const DevT
         n = x.n[c];
     }
     uint32_t grid = std::min<uint32_t>(n, uint32_t(device_sm_count()) * variant_occupancy(v));
-    return launch_pdl(kVariants[v].fn, grid, uint32_t(kVariants[v].threads), 0, stream, p, sg, t, n, rows, bs);
+    return launch_pdl(kVariants[v].fn, grid, uint32_t(kVariants[v].threads), 0, stream, p, sg, t, n, rows, split, bs);
 }
 }  // namespace
 
 const char* gemm_variant_name(int v) { return (v >= 0 && v < N_GEMM_VARIANTS) ? kVariants[v].name : "?"; }
 
 cudaError_t launch_gemm(GemmDev const& d, Bases const& bs, cudaStream_t stream) {
-    return launch_variant(d.var, d.p, d.s, d.t, d.n, d.x, d.r, bs, stream);
+    return launch_variant(d.var, d.p, d.s, d.t, d.n, d.x, d.r, d.split, bs, stream);
 }
 
 cudaError_t tune_program(DeviceProgram& prog, uint64_t in, uint64_t out, double* T, double* S, cudaStream_t stream) {
@@ -1432,9 +1685,12 @@ cudaError_t tune_program(DeviceProgram& prog, uint64_t in, uint64_t out, double*
         uint32_t n;
         TileLists x;
         const DevRow* r;
+        SplitArgs split;
         int* var;
-    } stages[2] = {{prog.d_p1, prog.d_s1, prog.d_t1, prog.n_t1, prog.x1, prog.d_r1, &prog.var1},
-                   {prog.d_p3, prog.d_s3, prog.d_t3, prog.n_t3, prog.x3, nullptr, &prog.var3}};
+    } stages[2] = {{prog.d_p1, prog.d_s1, prog.d_t1, prog.n_t1, prog.x1, prog.d_r1, {}, &prog.var1},
+                   {prog.d_p3, prog.d_s3, prog.d_t3, prog.n_t3, prog.x3, nullptr, {}, &prog.var3}};
+    if (prog.own3)
+        stages[1] = Stage{prog.f3.p, prog.f3.s, prog.f3.t, prog.f3.n, prog.f3.x, nullptr, prog.f3.split, &prog.var3};
     // stage 1 writes T, read by nothing else here; stage 3 reads S: both are timed on the
     // plan's current scratch contents (the kernels' speed does not depend on the values)
     // the clocks settle on a short run of the default variant first; then every
@@ -1445,13 +1701,13 @@ cudaError_t tune_program(DeviceProgram& prog, uint64_t in, uint64_t out, double*
     constexpr int ROUNDS = 4;
     for (auto& st : stages) {
         if (!st.n) continue;
-        for (int w = 0; w < 8 && e == cudaSuccess; ++w) e = launch_variant(0, st.p, st.s, st.t, st.n, st.x, st.r, bs, stream);
+        for (int w = 0; w < 8 && e == cudaSuccess; ++w) e = launch_variant(0, st.p, st.s, st.t, st.n, st.x, st.r, st.split, bs, stream);
         float best_v[N_GEMM_VARIANTS];
         for (int v = 0; v < N_GEMM_VARIANTS; ++v) best_v[v] = 1e30f;
         for (int round = 0; round < ROUNDS && e == cudaSuccess; ++round)
             for (int v = 0; v < N_GEMM_VARIANTS && e == cudaSuccess; ++v) {
                 cudaEventRecord(e0, stream);
-                e = launch_variant(v, st.p, st.s, st.t, st.n, st.x, st.r, bs, stream);
+                e = launch_variant(v, st.p, st.s, st.t, st.n, st.x, st.r, st.split, bs, stream);
                 cudaEventRecord(e1, stream);
                 if (e == cudaSuccess) e = cudaEventSynchronize(e1);
                 float ms = 0.f;
@@ -1526,7 +1782,7 @@ cudaError_t run_stages12(DeviceProgram const& prog, uint64_t in, uint64_t out, d
     bs.b[BUF_T] = reinterpret_cast<uint64_t>(T);
     bs.b[BUF_S] = reinterpret_cast<uint64_t>(S);
     bs.b[BUF_ABS] = 0;
-    launch_variant(prog.var1, prog.d_p1, prog.d_s1, prog.d_t1, prog.n_t1, prog.x1, prog.d_r1, bs, stream);
+    launch_variant(prog.var1, prog.d_p1, prog.d_s1, prog.d_t1, prog.n_t1, prog.x1, prog.d_r1, SplitArgs{}, bs, stream);
     cudaError_t e = run_sbuild(prog, T, S, stream);
     if (e != cudaSuccess) return e;
     return cudaGetLastError();
@@ -1549,12 +1805,18 @@ cudaError_t run_program(DeviceProgram const& prog, uint64_t in, uint64_t out, do
         if (ev) cudaEventRecord(ev[3], stream);
         return e != cudaSuccess ? e : cudaGetLastError();
     }
-    launch_variant(prog.var1, prog.d_p1, prog.d_s1, prog.d_t1, prog.n_t1, prog.x1, prog.d_r1, bs, stream);
+    launch_variant(prog.var1, prog.d_p1, prog.d_s1, prog.d_t1, prog.n_t1, prog.x1, prog.d_r1, SplitArgs{}, bs, stream);
     if (ev) cudaEventRecord(ev[1], stream);
     cudaError_t e = run_sbuild(prog, T, S, stream);
     if (e != cudaSuccess) return e;
     if (ev) cudaEventRecord(ev[2], stream);
-    launch_variant(prog.var3, prog.d_p3, prog.d_s3, prog.d_t3, prog.n_t3, prog.x3, nullptr, bs, stream);
+    if (prog.own3) {
+        GemmDev f3 = prog.f3;
+        f3.var = prog.var3;
+        if ((e = launch_gemm(f3, bs, stream)) != cudaSuccess) return e;
+    } else {
+        launch_variant(prog.var3, prog.d_p3, prog.d_s3, prog.d_t3, prog.n_t3, prog.x3, nullptr, SplitArgs{}, bs, stream);
+    }
     if (ev) cudaEventRecord(ev[3], stream);
     return cudaGetLastError();
 }

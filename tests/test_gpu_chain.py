@@ -1,11 +1,14 @@
 """Chained products (H·psi and boundary steps of plans with few terms per line, in one
-launch) on the device, against the oracle and against the GEMM stages (pinned variants), at sizes around the tiles: blocks of 1 to 33 rows (the chain
+launch) and K-split stage-3 problems on the device, against the oracle and against the
+GEMM stages (pinned variants), at sizes around the tiles: blocks of 1 to 33 rows (the chain
 takes up to 32; K1 and rows in blocks of 8, columns in tiles of 8, K2 in steps of 4)."""
 import numpy as np
 import pytest
 
 from dmrgb200 import engine as E
 from dmrgb200 import models as M
+from dmrgb200 import mps as S
+from dmrgb200 import su2u1 as SU
 from helpers import OracleChain, make_chain, random_psi
 
 import oracle as O
@@ -112,3 +115,27 @@ def test_chain_non_finite_boundary_stays_local():
     fine = np.isfinite(ref)
     assert not fine.all() and np.all(np.isfinite(y[fine]))
     assert _rel(y[fine], ref[fine]) <= TOL
+
+
+@pytest.mark.parametrize("L,m", [(8, 100), (10, 150)])
+def test_split_stage3_matches_oracle(L, m):
+    """Quantum chemistry in SU2U1 form: few output blocks with long K ranges, cut into parts
+    (K of up to a few thousand against parts of at least 48 steps of 16)."""
+    ctx = E.Context(0)
+    model = SU.quantum_chemistry(L, L, 0)
+    bonds = SU.synthetic_bonds(L, model.total_charge, m)
+    rng = np.random.default_rng(4)
+    tensors = S.random_mps(SU.PHYS, bonds, rng)
+    ch = OracleChain(model, bonds, tensors, L // 2 - 1)
+    plan, keep = _plan(ctx, ch)
+    x = rng.standard_normal(int(ch.sched.plan["in_size"]))
+    xd = E.to_device(x)
+    yd = torch.zeros_like(xd)
+    plan.hpsi(xd.data_ptr(), yd.data_ptr())
+    torch.cuda.synchronize()
+    y, ref = yd.cpu().numpy(), ch.hpsi(x)
+    # the lines' sums here have hundreds of terms: a thousand roundings
+    assert _rel(y, ref) <= 1e-12
+    plan.hpsi(xd.data_ptr(), yd.data_ptr())
+    torch.cuda.synchronize()
+    assert np.array_equal(yd.cpu().numpy(), y)  # parts are added in order, whichever arrives last
