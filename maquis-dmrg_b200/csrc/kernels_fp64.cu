@@ -404,52 +404,62 @@ __global__ void __launch_bounds__(NTHREADS, MINB) gemm_f64_grouped(const DevProb
 // the reference's axpy sequence), a cell without one writes zeros, so S needs
 // no separate clearing.  One warp per work item (a line and a chunk of SB_CHUNK
 // consecutive elements of its column-major walk): every lane owns SB_EPT elements
-// (lane + 32 u); the line's terms are read 32 at a time, one per lane, and handed
-// round by shuffles, so no block barrier is needed and the warps of a CTA, on
-// neighbouring chunks of one line, share its term list through L1.
+// (lane + 32 u).  A source is one run of T (leading dimension = rows), so the elements
+// of a term are its start plus fixed offsets: a term costs one broadcast read and a load
+// and a multiply-add per element, four terms in flight.  Only the store needs (i, c), by a
+// multiplication with the reciprocal of the row count.  (The terms handed round by
+// shuffles and a division per element took 71 instructions per element and warp on lines
+// of two terms, 18.8 us at the Hubbard middle of m = 1024 with the issue slots 45% busy.)
 constexpr int SB_EPT = 4, SB_CHUNK = 32 * SB_EPT;
 __global__ void __launch_bounds__(256) sbuild_lines(const DevSLine* __restrict__ lines,
                                                     const DevSTerm* __restrict__ terms,
                                                     const DevSItem* __restrict__ items, uint32_t n_items,
-                                                    double* __restrict__ S, const double* __restrict__ T) {
+                                                    double* __restrict__ S, const double* __restrict__ T, int more) {
+    const uint32_t lane = threadIdx.x & 31, stride = gridDim.x * (blockDim.x >> 5);
+    uint32_t it = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
+    // the tables are complete before the predecessor began; the next item's line is read
+    // while this one's sources are
+    DevSItem I{}, In{};
+    DevSLine L{};
+    if (it < n_items) I = items[it];
+    if (it + stride < n_items) In = items[it + stride];
+    if (it < n_items) L = lines[I.group];
     wait_for_predecessor();
-    const uint32_t lane = threadIdx.x & 31, wpb = blockDim.x >> 5;
-    for (uint32_t it = blockIdx.x * wpb + (threadIdx.x >> 5); it < n_items; it += gridDim.x * wpb) {
-        const DevSItem I = items[it];
-        const DevSLine L = lines[I.group];
-        const uint32_t n = L.rows * L.cols;
-        uint64_t toff[SB_EPT], soff[SB_EPT];
+    if (more) asm volatile("griddepcontrol.launch_dependents;" ::: "memory");  // see sbuild_groups
+    while (it < n_items) {
+        const uint32_t e0 = I.e0 + lane, n = L.rows * L.cols;
         bool in[SB_EPT];
         double v[SB_EPT];
 #pragma unroll
         for (int u = 0; u < SB_EPT; ++u) {
-            const uint32_t e = I.e0 + lane + 32u * u;
-            in[u] = e < n;
-            const uint32_t c = in[u] ? e / L.rows : 0, i = in[u] ? e - c * L.rows : 0;
-            toff[u] = i + uint64_t(c) * L.ld_t;
-            soff[u] = L.s_base + i + uint64_t(c) * L.ld_s;
+            in[u] = e0 + 32u * u < n;
             v[u] = 0.0;
         }
-        for (uint32_t t0 = L.term_begin; t0 < L.term_end; t0 += 32) {
-            const uint32_t nt = min(32u, L.term_end - t0);
-            double my_a = 0.0;
-            uint64_t my_b = 0;
-            if (lane < nt) {
-                const DevSTerm tm = terms[t0 + lane];
-                my_a = tm.alpha;
-                my_b = tm.t_base;
-            }
-            for (uint32_t t = 0; t < nt; ++t) {
-                const double a = __shfl_sync(0xffffffffu, my_a, t);
-                const uint64_t b = __shfl_sync(0xffffffffu, my_b, t);
+        const double* Te = T + e0;
+#pragma unroll 4
+        for (uint32_t t = L.term_begin; t < L.term_end; ++t) {
+            const double2 raw = __ldg(reinterpret_cast<const double2*>(terms + t));
+            const double* src = Te + __double_as_longlong(raw.y);
 #pragma unroll
-                for (int u = 0; u < SB_EPT; ++u)
-                    if (in[u]) v[u] += a * T[b + toff[u]];
-            }
+            for (int u = 0; u < SB_EPT; ++u)
+                if (in[u]) v[u] = fma(raw.x, src[32 * u], v[u]);
         }
+        const DevSLine Lc = L;
+        it += stride;
+        I = In;
+        if (it < n_items) L = lines[I.group];
+        if (it + stride < n_items) In = items[it + stride];
+        // column of element e: e / rows as the high word of e * (2^32 / rows + 1), exact while
+        // e * rows < 2^32
+        const uint32_t magic = 0xFFFFFFFFu / Lc.rows + 1u;
+        const bool small = uint64_t(n) * Lc.rows < (1ull << 32) && Lc.rows > 1;
+        double* dst = S + Lc.s_base;
 #pragma unroll
         for (int u = 0; u < SB_EPT; ++u)
-            if (in[u]) S[soff[u]] = v[u];
+            if (in[u]) {
+                const uint32_t e = e0 + 32u * u, c = small ? __umulhi(e, magic) : e / Lc.rows;
+                dst[(e - c * Lc.rows) + uint64_t(c) * Lc.ld_s] = v[u];
+            }
     }
 }
 
@@ -598,13 +608,20 @@ template <int NL>
 __global__ void __launch_bounds__(32 * SGB_WARPS, SgbShape<NL>::MINB)
     sbuild_groups(const DevSGroup* __restrict__ groups, const DevSItem* __restrict__ items, uint32_t n_items,
                   const uint64_t* __restrict__ ent_t, const double* __restrict__ ent_a, double* __restrict__ S,
-                  const double* __restrict__ T, int* err, unsigned long long wait_ns) {
+                  const double* __restrict__ T, int* err, unsigned long long wait_ns, int after_sbuild, int more) {
     using namespace async;
     constexpr int SGB_STAGES = SgbShape<NL>::STAGES;
     extern __shared__ __align__(16) unsigned char sgb_smem_raw[];
     const uint32_t lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     SgbRing<SGB_STAGES>& R = reinterpret_cast<SgbRing<SGB_STAGES>*>(sgb_smem_raw)[warp];
-    wait_for_predecessor();
+    // The launches of one S build write different parts of S from the same T.  The first waits
+    // for stage 1 and only then lets the next start (launch_dependents, where more follow), so a
+    // later one (after another of the S build) finds T complete and fills the SMs its
+    // predecessor's last CTAs leave; its own wait, at its end, keeps completion in stream order.
+    // At L = 12, m = 300 in quantum chemistry the three launches take 245 us instead of 330.  The
+    // last one lets nothing start early: stage 3's CTAs would hold SMs and wait.
+    if (!after_sbuild) wait_for_predecessor();
+    if (more) asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
     if (lane == 0) {
         for (int i = 0; i < SGB_STAGES; ++i) mbar_init(&R.full[i], 1);
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
@@ -626,6 +643,7 @@ __global__ void __launch_bounds__(32 * SGB_WARPS, SgbShape<NL>::MINB)
             }
         }
     }
+    if (after_sbuild) wait_for_predecessor();
 }
 
 // Register-resident DMMA loop for the FP64 tensor-core rate (calibration).
@@ -1733,12 +1751,16 @@ cudaError_t run_sbuild(DeviceProgram const& prog, double* T, double* S, cudaStre
         cudaError_t e = launch_pdl(sbuild_lines, grid, 256, 0, stream, static_cast<const DevSLine*>(prog.d_lines),
                                    static_cast<const DevSTerm*>(prog.d_terms),
                                    static_cast<const DevSItem*>(prog.d_litems), prog.n_litems, S,
-                                   static_cast<const double*>(T));
+                                   static_cast<const double*>(T), prog.n_gitems ? 1 : 0);
         if (e != cudaSuccess) return e;
     }
     // the items of groups of up to 8 lines come first (prog.n_gitems8 of them)
-    auto groups_launch = [&](auto kernel, size_t smem, int minb, const DevSItem* items, uint32_t n) -> cudaError_t {
+    int after = prog.n_litems ? 1 : 0;
+    auto groups_launch = [&](auto kernel, size_t smem, int minb, const DevSItem* items, uint32_t n,
+                             int more) -> cudaError_t {
         if (!n) return cudaSuccess;
+        const int after_sbuild = after;
+        after = 1;
         cudaError_t ea = ensure_smem_limit(reinterpret_cast<const void*>(kernel), int(smem));
         if (ea != cudaSuccess) return ea;
         // SGB_WARPS warps per CTA, minb CTAs per SM resident
@@ -1746,14 +1768,15 @@ cudaError_t run_sbuild(DeviceProgram const& prog, double* T, double* S, cudaStre
         return launch_pdl(kernel, grid, 32 * SGB_WARPS, smem, stream, static_cast<const DevSGroup*>(prog.d_groups),
                           items, n, static_cast<const uint64_t*>(prog.d_gent_t),
                           static_cast<const double*>(prog.d_gent_a), S, static_cast<const double*>(T), prog.d_err,
-                          wait_limit_ns());
+                          wait_limit_ns(), after_sbuild, more);
     };
     if (prog.n_gitems) {
         const DevSItem* items = static_cast<const DevSItem*>(prog.d_gitems);
-        cudaError_t e = groups_launch(sbuild_groups<8>, sgb_smem<8>(), SgbShape<8>::MINB, items, prog.n_gitems8);
+        cudaError_t e = groups_launch(sbuild_groups<8>, sgb_smem<8>(), SgbShape<8>::MINB, items, prog.n_gitems8,
+                                      prog.n_gitems > prog.n_gitems8 ? 1 : 0);
         if (e != cudaSuccess) return e;
         e = groups_launch(sbuild_groups<SG_LINES>, sgb_smem<SG_LINES>(), SgbShape<SG_LINES>::MINB,
-                          items + prog.n_gitems8, prog.n_gitems - prog.n_gitems8);
+                          items + prog.n_gitems8, prog.n_gitems - prog.n_gitems8, 0);
         if (e != cudaSuccess) return e;
     }
     return cudaGetLastError();
