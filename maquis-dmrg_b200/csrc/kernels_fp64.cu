@@ -51,6 +51,19 @@ __device__ __forceinline__ void dmma(double& c0, double& c1, double a, double b)
                  : "d"(a), "d"(b));
 }
 
+// 16 x 8 x 8 and 16 x 8 x 4 forms (rows g and g + 8 of A and C in one lane; k = q, q + 4)
+__device__ __forceinline__ void dmma16x8(double (&c)[4], const double (&a)[4], double b0, double b1) {
+    asm volatile(
+        "mma.sync.aligned.m16n8k8.row.col.f64.f64.f64.f64 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%0,%1,%2,%3};\n"
+        : "+d"(c[0]), "+d"(c[1]), "+d"(c[2]), "+d"(c[3])
+        : "d"(a[0]), "d"(a[1]), "d"(a[2]), "d"(a[3]), "d"(b0), "d"(b1));
+}
+__device__ __forceinline__ void dmma16x4(double (&c)[4], double a0, double a1, double b) {
+    asm volatile("mma.sync.aligned.m16n8k4.row.col.f64.f64.f64.f64 {%0,%1,%2,%3}, {%4,%5}, {%6}, {%0,%1,%2,%3};\n"
+                 : "+d"(c[0]), "+d"(c[1]), "+d"(c[2]), "+d"(c[3])
+                 : "d"(a0), "d"(a1), "d"(b));
+}
+
 // 8-byte asynchronous global->shared copy; src_bytes = 0 writes a zero (out-of-range element).
 __device__ __forceinline__ void cp_async8(double* smem, const double* gmem, bool valid) {
     unsigned saddr = static_cast<unsigned>(__cvta_generic_to_shared(smem));
@@ -523,13 +536,13 @@ __device__ __forceinline__ bool sgb_item(SgbRing<SGB_STAGES>& R, DevSGroup const
     using namespace async;
     const uint32_t n = G.rows * G.cols, cnt = min(uint32_t(SG_CHUNK), n - e0);
     const uint32_t k0 = G.ent_begin, k1 = G.ent_end;
-    constexpr int MT = SG_CHUNK / 8, NT = NL / 8;  // m8n8k4 tiles: elements x lines
+    constexpr int MT = SG_CHUNK / 16, NT = NL / 8;  // m16n8 tiles: elements x lines
     const uint32_t g = lane >> 2, q = lane & 3;
-    double acc[MT][NT][2];
+    double acc[MT][NT][4];
 #pragma unroll
     for (int i = 0; i < MT; ++i)
 #pragma unroll
-        for (int j = 0; j < NT; ++j) acc[i][j][0] = acc[i][j][1] = 0.0;
+        for (int j = 0; j < NT; ++j) acc[i][j][0] = acc[i][j][1] = acc[i][j][2] = acc[i][j][3] = 0.0;
     // every lane: the stage of sources kb .. kb + SGB_NC - 1 (those below k1)
     auto fill = [&](uint32_t kb) {
         const uint32_t slot = issued % SGB_STAGES, nc = min(uint32_t(SGB_NC), k1 - kb);
@@ -560,47 +573,55 @@ __device__ __forceinline__ bool sgb_item(SgbRing<SGB_STAGES>& R, DevSGroup const
         const bool ok = mbar_wait_suspend(&R.full[slot], (consumed / SGB_STAGES) & 1u, err, wait_ns);
         if (__any_sync(0xffffffffu, !ok)) return false;
         const uint32_t nc = min(uint32_t(SGB_NC), k1 - kb);
-        // D (elements x lines) += T (elements x 4 sources) * alpha (4 sources x lines) per
-        // K step of four sources (a group's sources are padded to a multiple of four, so a
-        // stage holds one or two whole steps); the alphas of both steps are read first
-        double b[SGB_NC / 4][NT];
+        // D (elements x lines) += T (elements x sources) * alpha (sources x lines): a whole
+        // stage of eight sources per DMMA, or its first four (a group's sources are padded to
+        // a multiple of four)
+        const double* r0 = R.rows[slot][q] + R.shift[slot][q] + g;
+        if (nc == uint32_t(SGB_NC)) {
+            const double* r1 = R.rows[slot][q + 4] + R.shift[slot][q + 4] + g;
+            double b0[NT], b1[NT];
 #pragma unroll
-        for (int ks = 0; ks < SGB_NC / 4; ++ks) {
-            const uint32_t c = uint32_t(ks * 4) + q;
-#pragma unroll
-            for (int j = 0; j < NT; ++j) b[ks][j] = c < nc ? R.alpha[slot][c][j * 8 + g] : 0.0;
-        }
-#pragma unroll
-        for (int ks = 0; ks < SGB_NC / 4; ++ks) {
-            if (uint32_t(ks * 4) >= nc) break;
-            const uint32_t c = uint32_t(ks * 4) + q;
-            const bool live = c < nc;
-            const double* row = R.rows[slot][c] + R.shift[slot][c] + g;
+            for (int j = 0; j < NT; ++j) {
+                b0[j] = R.alpha[slot][q][j * 8 + g];
+                b1[j] = R.alpha[slot][q + 4][j * 8 + g];
+            }
 #pragma unroll
             for (int i = 0; i < MT; ++i) {
-                const double a = live ? row[i * 8] : 0.0;
+                const double a[4] = {r0[i * 16], r0[i * 16 + 8], r1[i * 16], r1[i * 16 + 8]};
 #pragma unroll
-                for (int j = 0; j < NT; ++j) dmma(acc[i][j][0], acc[i][j][1], a, b[ks][j]);
+                for (int j = 0; j < NT; ++j) dmma16x8(acc[i][j], a, b0[j], b1[j]);
+            }
+        } else {
+            double b0[NT];
+#pragma unroll
+            for (int j = 0; j < NT; ++j) b0[j] = R.alpha[slot][q][j * 8 + g];
+#pragma unroll
+            for (int i = 0; i < MT; ++i) {
+                const double a0 = r0[i * 16], a1 = r0[i * 16 + 8];
+#pragma unroll
+                for (int j = 0; j < NT; ++j) dmma16x4(acc[i][j], a0, a1, b0[j]);
             }
         }
         ++consumed;
         __syncwarp();  // every lane's reads of this slot are done before it is refilled
     }
 #pragma unroll
-    for (int i = 0; i < MT; ++i) {
-        const uint32_t e = e0 + uint32_t(i * 8) + g;
-        if (e >= n) continue;
-        const uint32_t col = e / G.rows, r = e - col * G.rows;
-        double* dst = S + G.s_base + r + uint64_t(col) * G.ld_s;
+    for (int i = 0; i < MT; ++i)
 #pragma unroll
-        for (int j = 0; j < NT; ++j)
+        for (int r2 = 0; r2 < 2; ++r2) {
+            const uint32_t e = e0 + uint32_t(i * 16 + r2 * 8) + g;
+            if (e >= n) continue;
+            const uint32_t col = e / G.rows, r = e - col * G.rows;
+            double* dst = S + G.s_base + r + uint64_t(col) * G.ld_s;
 #pragma unroll
-            for (int h = 0; h < 2; ++h) {
-                const uint32_t line = uint32_t(j * 8) + 2u * q + uint32_t(h);
-                if (line < G.nlines)
-                    dst[uint64_t(line) * G.line_stride] = ((G.mask >> line) & 1u) ? acc[i][j][h] : 0.0;
-            }
-    }
+            for (int j = 0; j < NT; ++j)
+#pragma unroll
+                for (int h = 0; h < 2; ++h) {
+                    const uint32_t line = uint32_t(j * 8) + 2u * q + uint32_t(h);
+                    if (line < G.nlines)
+                        dst[uint64_t(line) * G.line_stride] = ((G.mask >> line) & 1u) ? acc[i][j][2 * r2 + h] : 0.0;
+                }
+        }
     return true;
 }
 
