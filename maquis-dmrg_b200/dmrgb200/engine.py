@@ -169,10 +169,12 @@ def schedule_right_step(phys, left, right, mpo: MPOHandle, R: BIndex, symmetric=
 # ---- device side --------------------------------------------------------------------
 
 def _view(addresses: np.ndarray):
-    arr = (C.c_void_p * max(len(addresses), 1))(*[int(a) if a else None for a in addresses])
+    """Boundary view over an array of addresses (0: no storage); the array is returned to be
+    kept alive as long as the view."""
+    arr = np.ascontiguousarray(addresses, dtype=np.uint64)
     v = capi.BoundaryView()
-    v.n_cohorts = len(addresses)
-    v.cohort_ptr = C.cast(arr, C.POINTER(C.c_void_p))
+    v.n_cohorts = len(arr)
+    v.cohort_ptr = C.cast(arr.ctypes.data, C.POINTER(C.c_void_p))
     return v, arr
 
 
