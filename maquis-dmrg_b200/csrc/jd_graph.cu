@@ -9,17 +9,17 @@
 //
 // jd_step is one cooperative launch of one CTA per SM.  Every thread owns the same
 // elements of all vectors throughout and keeps the target (t, u, uA) in registers; what
-// the CTAs exchange are the inner products: each CTA publishes its partial sums, a grid
-// barrier follows, and every CTA adds all partials in the same order, so all hold the
-// same coefficients without a second exchange, and a solve is bitwise reproducible.
-// What bounds it are those barriers (iteration k has k + 4 of them, 2k + 5 with
-// refinement) and the chain of rotations of the k x k eigenproblem, which every CTA
-// solves for itself; as separate launches, one per inner product and vector operation
-// (about 30 per iteration), it was the launches and their drains.
+// the CTAs exchange are the inner products: each CTA publishes its partial sums, every CTA
+// waits for all of them and adds them in the same order, so all hold the same coefficients
+// without a second exchange, and a solve is bitwise reproducible.  What bounds it are those
+// exchanges (iteration k has k + 4 of them, 2k + 5 with refinement) and the chain of
+// rotations of the k x k eigenproblem, which every CTA solves for itself; as separate
+// launches, one per inner product and vector operation (about 30 per iteration), it was
+// the launches and their drains.
 //
 // Each body sets the WHILE condition to 0 first and sets it back to 1 only at its end,
 // after incrementing the iteration count, so the loop ends after at most max_iter bodies
-// whatever the data.  The wait at a grid barrier is bounded (2 s): a CTA that gives up
+// whatever the data.  The wait for the other CTAs' sums is bounded (2 s): a CTA that gives up
 // records it, every later step returns at once and the solve reports DMRGB200_TIMEOUT.
 #include <cuda_runtime.h>
 
@@ -45,8 +45,8 @@ constexpr int MAXO = 8;        // orthogonal vectors bound
 constexpr int EPT = 4;         // elements per thread kept in registers
 
 struct JdState {
-    unsigned long long barrier;  // arrivals at grid barriers since the solve began
-    int iter, done, status, converged;  // status: 1 vanished direction, 2 barrier wait ran out
+    unsigned phase;              // exchanges since the solve began
+    int iter, done, status, converged;  // status: 1 vanished direction, 2 a wait ran out
     double theta, rnorm;
     double oo[MAXO];       // <o_i, o_i>
     double M[MAXK * MAXK]; // projected matrix, column-major, leading dimension MAXK
@@ -58,7 +58,7 @@ struct JdArgs {
     int max_iter, n_ortho;
     double tol;
     JdState* st;
-    double* partial;      // [2][MAXK][grid] partial sums of the CTAs
+    double* partial;      // [2][MAXK][grid] places of the CTAs' partial sums, 16 bytes each
     cudaGraphConditionalHandle cond;
 };
 
@@ -109,65 +109,97 @@ struct StepShared {
     int failed;
 };
 
-// Sums of nv per-thread values over the grid: warp trees, the CTA's partial sums to
-// global memory, a grid barrier, then warp w of every CTA adds value w over all CTAs (the
-// same order everywhere).  Results in sh.sum[0, nv).  `val(k, v)` gives the thread's values
-// k .. k + 3 (those below nv count), four at a time so that their loads overlap.  False when
-// the barrier's wait ran out.
+// A place of an exchange: a CTA's partial sum and the number of the exchange it belongs to,
+// stored and read as one 128-bit word.
+__device__ __forceinline__ void place_store(double* at, double v, unsigned long long tag) {
+    asm volatile(
+        "{\n\t.reg .b128 w;\n\tmov.b128 w, {%1, %2};\n\tst.relaxed.gpu.global.b128 [%0], w;\n\t}" ::"l"(at),
+        "l"(__double_as_longlong(v)), "l"(tag)
+        : "memory");
+}
+__device__ __forceinline__ void place_load(const double* at, unsigned long long& v, unsigned long long& tag) {
+    asm volatile("{\n\t.reg .b128 w;\n\tld.relaxed.gpu.global.b128 w, [%2];\n\tmov.b128 {%0, %1}, w;\n\t}"
+                 : "=l"(v), "=l"(tag)
+                 : "l"(at)
+                 : "memory");
+}
+
+// Sums of nv per-thread values over the grid: warp trees, the CTA's partial sums to global
+// memory, then warp w of every CTA reads value w of all CTAs (waiting for those of an earlier
+// exchange) and adds them, in the same order everywhere.  Results in sh.sum[0, nv).
+// `val(k, v)` gives the thread's values k .. k + 3 (those below nv count), four at a time so
+// that their loads overlap.  False when a wait ran out.
+//
+// The sum and its tag travel in one word, so it is its own flag: no counter, no fence, one trip
+// through L2 (6 us per exchange with fences or a counted barrier).  Exchange `phase` uses the
+// places phase % 2: a CTA stores there again two exchanges later, when it has seen every other
+// CTA's sum of the exchange between, which each of them stored after it had read this one.
 template <class F>
 __device__ bool grid_sums(JdArgs const& a, StepShared& sh, int nv, unsigned& phase, F&& val) {
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    double* part = a.partial + uint64_t(phase & 1u) * MAXK * gridDim.x;
-    ++phase;
+    double* part = a.partial + uint64_t(phase & 1u) * 2 * MAXK * gridDim.x;
+    const unsigned long long tag = ++phase;
     for (int k = 0; k < nv; k += 4) {
         double v[4] = {0.0, 0.0, 0.0, 0.0};
         val(k, v);
+        if (nv - k == 1) {
 #pragma unroll
-        for (int o = 16; o > 0; o >>= 1)
+            for (int o = 16; o > 0; o >>= 1) v[0] += __shfl_xor_sync(0xffffffffu, v[0], o);
+        } else {
 #pragma unroll
-            for (int j = 0; j < 4; ++j) v[j] += __shfl_xor_sync(0xffffffffu, v[j], o);
+            for (int o = 16; o > 0; o >>= 1)
+#pragma unroll
+                for (int j = 0; j < 4; ++j) v[j] += __shfl_xor_sync(0xffffffffu, v[j], o);
+        }
         if (lane == 0)
 #pragma unroll
             for (int j = 0; j < 4; ++j)
                 if (k + j < nv) sh.red[warp][k + j] = v[j];
     }
+    if (threadIdx.x == 0) sh.failed = 0;
     __syncthreads();
     if (warp < nv) {
         double v = sh.red[lane][warp];
 #pragma unroll
         for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
-        if (lane == 0) __stcg(part + uint64_t(warp) * gridDim.x + blockIdx.x, v);
-    }
-    __syncthreads();
-    if (threadIdx.x == 0) {
-        // arrive, then wait until every CTA of this generation has (each CTA arrives once per
-        // generation, so the arrival's number tells the generation)
-        __threadfence();
-        const unsigned long long target = (atomicAdd(&a.st->barrier, 1ull) / gridDim.x + 1ull) * gridDim.x;
+        double* row = part + 2 * uint64_t(warp) * gridDim.x;
+        if (lane == 0) place_store(row + 2 * blockIdx.x, v, tag);
         const unsigned long long t0 = async::global_ns();
-        unsigned long long seen;
-        sh.failed = 0;
-        for (;;) {
-            asm volatile("ld.acquire.gpu.u64 %0, [%1];" : "=l"(seen) : "l"(&a.st->barrier) : "memory");
-            if (seen >= target) break;
-            if (async::global_ns() - t0 > async::WAIT_LIMIT_NS) {
-                sh.failed = 1;
-                atomicExch(&a.st->status, 2);
-                break;
+        v = 0.0;
+        bool ok = true;
+        for (unsigned b0 = lane; b0 < gridDim.x; b0 += 32 * 5) {
+            // this lane's places, all read at once until each carries the tag
+            unsigned long long x[5], y[5];
+            for (;;) {
+                bool all = true;
+#pragma unroll
+                for (int j = 0; j < 5; ++j) {
+                    x[j] = 0ull;
+                    y[j] = tag;
+                    if (b0 + 32 * j < gridDim.x) place_load(row + 2 * (b0 + 32 * j), x[j], y[j]);
+                }
+#pragma unroll
+                for (int j = 0; j < 5; ++j) all = all && y[j] == tag;
+                if (all) break;
+                if (async::global_ns() - t0 > async::WAIT_LIMIT_NS) {
+                    ok = false;
+                    break;
+                }
             }
+#pragma unroll
+            for (int j = 0; j < 5; ++j) v += __longlong_as_double(x[j]);  // 0 past the last CTA
         }
-    }
-    __syncthreads();
-    if (sh.failed) return false;
-    if (warp < nv) {
-        double v = 0.0;
-        for (unsigned b = lane; b < gridDim.x; b += 32) v += __ldcg(part + uint64_t(warp) * gridDim.x + b);
+        if (!ok) {
+            sh.failed = 1;
+            atomicExch(&a.st->status, 2);
+        }
+        __syncwarp();
 #pragma unroll
         for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
         if (lane == 0) sh.sum[warp] = v;
     }
     __syncthreads();
-    return true;
+    return !sh.failed;
 }
 
 // Project the orthogonal vectors out of x: x -= <o_i, x> / <o_i, o_i> o_i in turn.
@@ -188,38 +220,53 @@ __device__ bool project(JdArgs const& a, StepShared& sh, unsigned& phase, Own<RE
 // normalisation; also left in the H psi input.
 template <bool REG>
 __device__ bool basis_vector(JdArgs const& a, StepShared& sh, unsigned& phase, Own<REG>& t, int it) {
+    // v: the basis vector whose coefficient comes next, w: the one after it (read ahead of the
+    // exchange that gives the coefficient)
+    double v[REG ? EPT : 1], w[REG ? EPT : 1];
+    auto fetch = [&](double(&d)[REG ? EPT : 1], int j) {
+        if (REG && j < it) each<REG>(a, [&](int e, uint64_t k) { d[e] = V(a, j)[k]; });
+    };
+    auto basis = [&](double(&d)[REG ? EPT : 1], int j, int e, uint64_t k) { return REG ? d[e] : V(a, j)[k]; };
+    fetch(v, 0);
+    fetch(w, 1);
     // tau^2 = <t, t> and the first coefficient in one exchange
     double tt = 0.0, p = 0.0;
     each<REG>(a, [&](int e, uint64_t k) {
         const double x = t.get(e, k);
         tt += x * x;
-        if (it > 0) p += V(a, 0)[k] * x;
+        if (it > 0) p += basis(v, 0, e, k) * x;
     });
-    if (!grid_sums(a, sh, it > 0 ? 2 : 1, phase, [&](int, double* v) {
-            v[0] = tt;
-            v[1] = p;
-        })) return false;
+    if (!grid_sums(a, sh, it > 0 ? 2 : 1, phase, [&](int, double* s) {
+            s[0] = tt;
+            s[1] = p;
+        }))
+        return false;
     const double tau = sqrt(sh.sum[0]);
     double nn = sh.sum[0], c = it > 0 ? sh.sum[1] : 0.0;
     for (int pass = 0; it > 0 && pass < 2; ++pass) {
         if (pass == 1) {
             if (!(sqrt(nn) < 0.25 * tau)) break;
+            fetch(v, 0);
+            fetch(w, 1);
             p = 0.0;
-            each<REG>(a, [&](int e, uint64_t k) { p += V(a, 0)[k] * t.get(e, k); });
-            if (!grid_sums(a, sh, 1, phase, [&](int, double* v) { v[0] = p; })) return false;
+            each<REG>(a, [&](int e, uint64_t k) { p += basis(v, 0, e, k) * t.get(e, k); });
+            if (!grid_sums(a, sh, 1, phase, [&](int, double* s) { s[0] = p; })) return false;
             c = sh.sum[0];
         }
         // t -= c V(j) and, in the same pass over t, the next coefficient (or |t|^2 at the end)
         for (int j = 0; j < it; ++j) {
-            const double* v = V(a, j);
-            const double* w = j + 1 < it ? V(a, j + 1) : nullptr;
+            const bool more = j + 1 < it;
             p = 0.0;
             each<REG>(a, [&](int e, uint64_t k) {
-                const double x = t.get(e, k) - c * v[k];
+                const double x = t.get(e, k) - c * basis(v, j, e, k);
                 t.set(e, k, x);
-                p += (w ? w[k] : x) * x;
+                p += (more ? basis(w, j + 1, e, k) : x) * x;
             });
-            if (!grid_sums(a, sh, 1, phase, [&](int, double* v) { v[0] = p; })) return false;
+            if (REG)
+#pragma unroll
+                for (int e = 0; e < (REG ? EPT : 1); ++e) v[e] = w[e];
+            fetch(w, j + 2);
+            if (!grid_sums(a, sh, 1, phase, [&](int, double* s) { s[0] = p; })) return false;
             c = nn = sh.sum[0];
         }
     }
@@ -237,13 +284,36 @@ __device__ bool basis_vector(JdArgs const& a, StepShared& sh, unsigned& phase, O
         a.st->done = 1;
     }
     const double inv = vanished ? 0.0 : 1.0 / tn;
-    double *in = Tv(a), *v = V(a, it);
+    double *in = Tv(a), *out = V(a, it);
     each<REG>(a, [&](int e, uint64_t k) {
         const double x = t.get(e, k) * inv;
         in[k] = x;
-        v[k] = x;
+        out[k] = x;
     });
     return !vanished;
+}
+
+// 1 / sqrt(w) to rounding: rsqrt and a Newton step
+__device__ __forceinline__ double recip_sqrt(double w) {
+    const double r = rsqrt(w);
+    return fma(0.5 * r, fma(-(w * r), r, 1.0), r);
+}
+
+// Rotation of a pair, tan(2x) = h / d (h = 2 a_pq, d = a_qq - a_pp), the smaller angle:
+// cos(2x) = |d| / sqrt(d^2 + h^2), c^2 = (1 + cos(2x)) / 2 and s = sin(2x) / (2 c), two reciprocal
+// square roots in sequence instead of two square roots and three divisions.  (The tangent in
+// single precision and two Newton steps is shorter still, but takes two sweeps more.)
+__device__ __forceinline__ void rotation(double d, double h, double& c, double& s) {
+    const double w = fma(d, d, h * h);
+    if (d != 0.0 && w > 1e-280 && w < 1e280) {
+        const double r = recip_sqrt(w), c2 = fma(0.5 * fabs(d), r, 0.5), ic = recip_sqrt(c2);
+        c = c2 * ic;
+        s = copysign(0.5, d) * h * r * ic;
+    } else {
+        const double tau = d / h, t = (tau >= 0 ? 1.0 : -1.0) / (fabs(tau) + sqrt(1.0 + tau * tau));
+        c = 1.0 / sqrt(1.0 + t * t);
+        s = t * c;
+    }
 }
 
 // Smallest eigenpair of the leading k x k block of M by cyclic Jacobi, one warp, from the
@@ -255,6 +325,7 @@ __device__ bool basis_vector(JdArgs const& a, StepShared& sh, unsigned& phase, O
 // square root).
 __device__ void ritz(StepShared& sh, int k) {
     const int lane = threadIdx.x & 31;
+    const int inv = 65535 / k + 1;  // e / k = (e * inv) >> 16 for e < 512, k <= 32
     for (int e = lane; e < k * k; e += 32) sh.Z[e / k][e % k] = e / k == e % k ? 1.0 : 0.0;
     __syncwarp();
     for (int sweep = 0; sweep < 100; ++sweep) {
@@ -284,11 +355,7 @@ __device__ void ritz(StepShared& sh, int k) {
                 if (drop) {
                     sh.A[p][q] = sh.A[q][p] = 0.0;
                 } else if (apq != 0.0) {
-                    const double d = aqq - app, h = 2.0 * apq;
-                    const double t = d == 0.0 ? 1.0 : h / (d + copysign(sqrt(fma(d, d, h * h)), d));
-                    const double w = fma(t, t, 1.0), c0 = rsqrt(w);
-                    c = fma(0.5 * c0, fma(-(w * c0), c0, 1.0), c0);  // to rounding
-                    s = t * c;
+                    rotation(aqq - app, 2.0 * apq, c, s);
                     any = true;
                 }
                 sh.cs[lane][0] = c;
@@ -296,9 +363,10 @@ __device__ void ritz(StepShared& sh, int k) {
             }
             if (!__any_sync(0xffffffffu, any)) continue;
             __syncwarp();
-            // A <- A J and Z <- Z J, then A <- J^T A
+            // A <- A J and Z <- Z J, then A <- J^T A: one row (column) of one pair per lane at a
+            // time, so that the lanes' reads do not wait for each other's writes
             for (int e = lane; e < np * k; e += 32) {
-                const int r = e % k, x = e / k, p = p0 + x, q = sum - p;
+                const int x = (e * inv) >> 16, r = e - x * k, p = p0 + x, q = sum - p;
                 const double c = sh.cs[x][0], s = sh.cs[x][1];
                 const double ap = sh.A[r][p], aq = sh.A[r][q], zp = sh.Z[r][p], zq = sh.Z[r][q];
                 sh.A[r][p] = c * ap - s * aq;
@@ -308,7 +376,7 @@ __device__ void ritz(StepShared& sh, int k) {
             }
             __syncwarp();
             for (int e = lane; e < np * k; e += 32) {
-                const int r = e % k, x = e / k, p = p0 + x, q = sum - p;
+                const int x = (e * inv) >> 16, r = e - x * k, p = p0 + x, q = sum - p;
                 const double c = sh.cs[x][0], s = sh.cs[x][1];
                 const double ap = sh.A[p][r], aq = sh.A[q][r];
                 sh.A[p][r] = c * ap - s * aq;
@@ -330,8 +398,8 @@ __device__ void ritz(StepShared& sh, int k) {
 template <bool REG>
 __global__ void __launch_bounds__(JT) jd_start(JdArgs a) {
     __shared__ StepShared sh;
-    unsigned phase = 0;
     JdState* st = a.st;
+    unsigned phase = st->phase;
     for (int i = 0; i < a.n_ortho; ++i) {
         Own<false> o;
         o.g = Ov(a, i);
@@ -348,7 +416,10 @@ __global__ void __launch_bounds__(JT) jd_start(JdArgs a) {
     each<REG>(a, [&](int e, uint64_t k) { t.set(e, k, Tv(a)[k]); });
     if (a.n_ortho > 0 && !project<REG>(a, sh, phase, t, a.n_ortho)) return;
     const bool ok = basis_vector<REG>(a, sh, phase, t, 0);
-    if (!ok && blockIdx.x == 0 && threadIdx.x == 0) cudaGraphSetConditional(a.cond, 0u);
+    if (blockIdx.x == 0 && threadIdx.x == 0) {
+        st->phase = phase;
+        if (!ok) cudaGraphSetConditional(a.cond, 0u);
+    }
 }
 
 // The part of an iteration after its H psi (y): projected matrix, Ritz pair, residual and
@@ -361,7 +432,7 @@ __global__ void __launch_bounds__(JT) jd_step(JdArgs a) {
     const bool lead = blockIdx.x == 0 && threadIdx.x == 0;
     if (lead) cudaGraphSetConditional(a.cond, 0u);
     if (st->status) return;
-    unsigned phase = 0;
+    unsigned phase = st->phase;
     // VA(it) = y; M(j, it) = <V(j), y>, j <= it
     Own<REG> y;
     y.g = VA(a, it);
@@ -423,7 +494,7 @@ __global__ void __launch_bounds__(JT) jd_step(JdArgs a) {
         })) return;
     const double rnorm = sqrt(sh.sum[0]), corr = sh.sum[1] / sh.sum[2];
     const bool conv = rnorm <= a.tol * fabs(theta) || rnorm < a.tol, done = conv || it + 1 >= a.max_iter;
-    // every CTA is past the barrier above, so none still reads st->iter
+    // every CTA's sums have arrived, so none still reads st->iter
     if (lead) {
         st->theta = theta;
         st->rnorm = rnorm;
@@ -437,7 +508,11 @@ __global__ void __launch_bounds__(JT) jd_step(JdArgs a) {
     }
     // t = -r + corr u (in place of r)
     each<REG>(a, [&](int e, uint64_t i) { ua.set(e, i, -ua.get(e, i) + corr * u.get(e, i)); });
-    if (basis_vector<REG>(a, sh, phase, ua, it + 1) && lead) cudaGraphSetConditional(a.cond, 1u);
+    const bool ok = basis_vector<REG>(a, sh, phase, ua, it + 1);
+    if (lead) {
+        st->phase = phase;
+        if (ok) cudaGraphSetConditional(a.cond, 1u);
+    }
 }
 
 }  // namespace
@@ -489,7 +564,7 @@ cudaError_t build_graph(JdGraph& g, dmrgb200_plan_t plan, cudaStream_t s) {
     const int nb = device_sm_count();  // one CTA per SM: all resident, as a cooperative launch needs
     if ((e = cudaMalloc(&g.vec, sizeof(double) * n * nslots)) != cudaSuccess) return e;
     if ((e = cudaMalloc(&g.st, sizeof(JdState))) != cudaSuccess) return e;
-    if ((e = cudaMalloc(&g.partial, sizeof(double) * 2 * nb * MAXK)) != cudaSuccess) return e;
+    if ((e = cudaMalloc(&g.partial, sizeof(double) * 4 * nb * MAXK)) != cudaSuccess) return e;
     // H psi writes only block elements: the padding of every slot stays zero
     if ((e = cudaMemset(g.vec, 0, sizeof(double) * n * nslots)) != cudaSuccess) return e;
     if ((e = cudaMemset(g.st, 0, sizeof(JdState))) != cudaSuccess) return e;
@@ -521,6 +596,8 @@ cudaError_t build_graph(JdGraph& g, dmrgb200_plan_t plan, cudaStream_t s) {
     // vectors of up to EPT elements per thread stay in registers between the passes
     const bool reg = n <= uint64_t(EPT) * JT * nb;
     if ((e = cudaMemsetAsync(g.st, 0, sizeof(JdState), s)) == cudaSuccess)
+        e = cudaMemsetAsync(g.partial, 0, sizeof(double) * 4 * nb * MAXK, s);  // tags start at 1
+    if (e == cudaSuccess)
         e = launch_cooperative(reg ? jd_start<true> : jd_start<false>, nb, a, s);
     cudaGraph_t captured = nullptr;
     const cudaError_t le = e;
@@ -620,7 +697,7 @@ dmrgb200_status solve_graph(dmrgb200_plan_t plan, void** cache, uint64_t n, cons
 #undef CK
     float ms = 0.f;
     cudaEventElapsedTime(&ms, g->e0, g->e1);
-    if (hs.status == 2) return noalloc_fail(DMRGB200_TIMEOUT, "solver: the wait at a grid barrier ran out");
+    if (hs.status == 2) return noalloc_fail(DMRGB200_TIMEOUT, "solver: the wait for an inner product ran out");
     if (hs.status) return noalloc_fail(DMRGB200_NUMERIC, "Davidson direction vanished");
     *energy = hs.theta;
     if (stats) {
