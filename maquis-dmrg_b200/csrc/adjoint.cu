@@ -559,9 +559,10 @@ cudaError_t run_adjoint(DeviceProgram const& fwd, AdjointProgram const& a, uint6
     const uint32_t sms = uint32_t(device_sm_count());
     cudaError_t e;
     if (!gx && !galpha) return cudaSuccess;
-    GemmDev d3 = a.d3, d1 = a.d1;  // the transposed stages use the forward stages' tuned variants
-    d3.var = fwd.var3;
-    d1.var = fwd.var1;
+    // the transposed stages use the forward stages' variants where those were tuned or pinned
+    GemmDev d3 = a.d3, d1 = a.d1;
+    d3.var = fwd.tuned ? fwd.var3 : gemm_default_variant(a.g3);
+    d1.var = fwd.tuned ? fwd.var1 : gemm_default_variant(a.g1);
     if ((e = launch_gemm(d3, bs, stream)) != cudaSuccess) return e;  // G into S
     if (galpha) {
         GemmDev f1;
@@ -571,7 +572,7 @@ cudaError_t run_adjoint(DeviceProgram const& fwd, AdjointProgram const& a, uint6
         f1.n = fwd.n_t1;
         f1.x = fwd.x1;
         f1.r = fwd.d_r1;
-        f1.var = fwd.var1;
+        f1.var = fwd.tuned ? fwd.var1 : gemm_default_variant(fwd.stage1);
         if ((e = launch_gemm(f1, bs, stream)) != cudaSuccess) return e;  // T = x-slices * R
         if (a.n_aterms) {
             uint32_t grid = std::min<uint32_t>((a.n_aterms + 7) / 8, sms * 8);

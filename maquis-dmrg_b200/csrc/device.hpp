@@ -307,6 +307,8 @@ const char* gemm_variant_name(int v);
 cudaError_t tune_program(DeviceProgram& prog, uint64_t in, uint64_t out, double* T, double* S, cudaStream_t stream);
 cudaError_t upload_gemm(GemmList const& gl, GemmDev& d);
 void free_gemm(GemmDev& d);
+// variant of a list that nobody timed
+int gemm_default_variant(GemmList const& gl);
 // one persistent grouped-GEMM launch over the tile list
 cudaError_t launch_gemm(GemmDev const& d, Bases const& bs, cudaStream_t stream);
 

@@ -1698,6 +1698,10 @@ cudaError_t launch_variant(int v, const DevProb* p, const DevSeg* sg, const DevT
 }
 }  // namespace
 
+// 64 x 64 tiles at three CTAs per SM where they fill the chip twice (SU2U1 L=16 m=512 stage 1,
+// 472 us against 536 for 32 x 64; on shorter lists the smaller tiles balance better)
+int gemm_default_variant(GemmList const& gl) { return gl.tiles_cls[2].size() >= 2 * 3 * 148 ? 6 : 0; }
+
 const char* gemm_variant_name(int v) { return (v >= 0 && v < N_GEMM_VARIANTS) ? kVariants[v].name : "?"; }
 
 cudaError_t launch_gemm(GemmDev const& d, Bases const& bs, cudaStream_t stream) {
