@@ -222,7 +222,8 @@ dmrgb200_status dmrgb200_hpsi_per_block(dmrgb200_plan_t plan, const double* x, d
  * per SM) is timed on the plan's stage-1 and stage-3 tile lists and the
  * fastest is kept per stage.  The first FP64 dmrgb200_hpsi / dmrgb200_solve of
  * a plan of at least 50 MFLOP per H·psi does this by itself (environment
- * DMRGB200_AUTOTUNE=0 keeps the default variant); this call re-tunes now, using x (in layout) and y (out
+ * DMRGB200_AUTOTUNE=0 keeps the default variant; plans of small blocks that run as chained
+ * products have no GEMM stages to tune); this call re-tunes now, using x (in layout) and y (out
  * layout, overwritten), and returns the chosen variant per stage.  No
  * counterpart in the reference (its cuBLAS calls are untuned). */
 dmrgb200_status dmrgb200_plan_autotune(dmrgb200_plan_t plan, const double* x, double* y, void* cuda_stream,
@@ -232,7 +233,8 @@ const char* dmrgb200_gemm_variant_name(int variant);
 int dmrgb200_gemm_variant_count(void);
 /* Pin the grouped-GEMM variant of stage 1 and of stage 3 of an H·psi plan (each 0 ..
  * dmrgb200_gemm_variant_count() - 1) instead of the autotuner's choice: later calls use
- * them and do not tune the plan (dmrgb200_plan_autotune re-tunes).  The sums are the same
+ * them and do not tune the plan (dmrgb200_plan_autotune re-tunes); a plan of small blocks,
+ * which otherwise runs as chained products in one launch, runs its stages from then on.  The sums are the same
  * for every variant up to the order of the K steps.  No counterpart in the reference. */
 dmrgb200_status dmrgb200_plan_set_gemm_variants(dmrgb200_plan_t plan, int32_t stage1, int32_t stage3);
 
@@ -322,7 +324,8 @@ dmrgb200_status dmrgb200_plan_set_slices(dmrgb200_plan_t plan, int slices);
  * dmrgb200_plan_stage_times synchronises the last recorded events and returns
  * the accumulated milliseconds and the number of timed calls; stage 0 = T
  * GEMMs (create_T), 1 = S build (create_s_r), 2 = cohort contraction
- * (contract).  Algorithmic flops per stage per call are returned in flops[3]. */
+ * (contract); a plan that runs as chained products (one launch) is timed whole as stage 2.
+ * Algorithmic flops per stage per call are returned in flops[3]. */
 dmrgb200_status dmrgb200_plan_set_timing(dmrgb200_plan_t plan, int enable);
 dmrgb200_status dmrgb200_plan_stage_times(dmrgb200_plan_t plan, double ms[3], uint64_t flops[3], uint64_t* calls);
 
