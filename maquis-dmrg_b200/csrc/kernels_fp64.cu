@@ -99,8 +99,8 @@ __device__ __forceinline__ int swz(int k) { return (k >> 2) & 3; }
 // problem are not copied: what the tile holds there only reaches outputs that are not
 // stored.  A whole K step has no per-copy conditions (about five instructions per copy
 // instead of ten: on blocks of 17 to 52 rows the copies' arithmetic is most of what the
-// kernel executes); the last one of a segment zero-fills its K rows past the end, up to the
-// DMMA step of four that is multiplied.
+// kernel executes); the last one of a segment zero-fills its K rows past the end, in the half
+// or the whole stage that is multiplied.
 struct CopyStream {
     const char* base;
     const char* safe;  // a readable address for copies that fetch nothing
@@ -125,7 +125,7 @@ __device__ __forceinline__ void issue_copies(double* tile, CopyStream& cs, uint3
                 for (int j = 0; j < NC; ++j, p += cs.jstride)
                     cp_async8_all(&tile[(cs.kt + j * KJ) * LD + (cs.r ^ ((t0 + ((j * KJ) >> 2)) & 3u))], p);
             } else {
-                const uint32_t kend = (krem + 3u) & ~3u;
+                const uint32_t kend = krem > uint32_t(BK_ / 2) ? BK_ : BK_ / 2;
 #pragma unroll
                 for (int j = 0; j < NC; ++j, p += cs.jstride) {
                     const uint32_t k = cs.kt + j * KJ;
@@ -145,7 +145,7 @@ __device__ __forceinline__ void issue_copies(double* tile, CopyStream& cs, uint3
 #pragma unroll
             for (int j = 0; j < NC; ++j, p += cs.jstride)
                 if ((cs.mask >> j) & 1u) cp_async8_all(dst + j * RJ, p);
-        } else if (cs.kt < ((krem + 3u) & ~3u)) {
+        } else if (cs.kt < (krem > uint32_t(BK_ / 2) ? BK_ : BK_ / 2)) {
 #pragma unroll
             for (int j = 0; j < NC; ++j, p += cs.jstride)
                 if ((cs.mask >> j) & 1u) cp_async8(dst + j * RJ, reinterpret_cast<const double*>(kok ? p : cs.safe), kok);
@@ -307,15 +307,15 @@ __global__ void __launch_bounds__(NTHREADS, MINB) gemm_f64_grouped(const DevProb
         const uint32_t M = pr.M, N = pr.N;
         const bool inside = tl.m0 + wm < M && tl.n0 + wn < N;  // any of this warp's tile
         for (uint32_t st = 0; st < tl.nsteps; ++st) {
+            const uint32_t kn = st_k[slot];  // written when the stage was issued, a barrier ago
             issue((slot + STAGES - 1) % STAGES);
             cp_async_commit();
             cp_async_wait<STAGES - 1>();
             __syncthreads();
-            // K steps of four past the segment's end are not multiplied, nor tiles of warps outside
-            // the problem; the unrolled forms keep the fragment reads ahead of the products (a
-            // condition per step of four costs more than it saves: Heisenberg m = 1024 stage 3
-            // 52 us instead of 44)
-            const uint32_t kn = (st_k[slot] + 3u) / 4u;
+            // the second half of a stage that holds at most half its K rows is not multiplied, nor
+            // tiles of warps outside the problem; unrolled forms keep the fragment reads ahead of the
+            // products (a condition per K step of four, or a form per count of them, costs more
+            // than it saves where a CTA has its SM to itself)
             if (inside) {
                 auto product = [&](auto steps) {
                     constexpr int KS = decltype(steps)::value;
@@ -332,10 +332,8 @@ __global__ void __launch_bounds__(NTHREADS, MINB) gemm_f64_grouped(const DevProb
                             for (int j = 0; j < NJ; ++j) dmma(acc[i][j][0], acc[i][j][1], a[i], b[j]);
                     }
                 };
-                if (kn == BK_ / 4) product(std::integral_constant<int, BK_ / 4>());
-                else if (kn == 1) product(std::integral_constant<int, 1>());
-                else if (BK_ > 8 && kn == 2) product(std::integral_constant<int, 2>());
-                else if (BK_ > 8 && kn == 3) product(std::integral_constant<int, 3>());
+                if (kn > uint32_t(BK_ / 2)) product(std::integral_constant<int, BK_ / 4>());
+                else if (kn) product(std::integral_constant<int, BK_ / 8>());
             }
             __syncthreads();
             slot = (slot + 1) % STAGES;
