@@ -211,8 +211,7 @@ __global__ void __launch_bounds__(NTHREADS, MINB) gemm_f64_grouped(const DevProb
                   "tile shape");
     __shared__ __align__(16) double As[STAGES][BK_][pitch<BM_>()];
     __shared__ __align__(16) double Bs[STAGES][BK_][pitch<BN_>()];
-    __shared__ uint32_t st_k[STAGES];  // K rows a stage holds
-    __shared__ uint32_t st_last;       // this tile's part arrived last (K-split problems)
+    __shared__ uint32_t st_last;  // this tile's part arrived last (K-split problems)
     wait_for_predecessor();
 
     const int tid = threadIdx.x;
@@ -268,28 +267,35 @@ __global__ void __launch_bounds__(NTHREADS, MINB) gemm_f64_grouped(const DevProb
         L.seg_end = pr.seg_end;
         enter_segment();
     };
-    auto issue = [&](int slot) {
-        if (!L.valid) return;
-        if (tid == 0) st_k[slot] = L.seg < L.seg_end ? min(L.krem, uint32_t(BK_)) : 0u;
+    // returns the K rows the stage holds
+    auto issue = [&](int slot) -> uint32_t {
+        if (!L.valid) return 0u;
+        uint32_t rows = 0;
         if (L.seg < L.seg_end) {  // an empty tile issues no copies
+            rows = min(L.krem, uint32_t(BK_));
             issue_copies<BM_, BK_, NTHREADS, pitch<BM_>()>(&As[slot][0][0], ca, L.krem);
             issue_copies<BN_, BK_, NTHREADS, pitch<BN_>()>(&Bs[slot][0][0], cb, L.krem);
             if (L.krem > uint32_t(BK_)) {
                 L.krem -= BK_;
-                return;
+                return rows;
             }
             ++L.seg;
             enter_segment();
-            if (L.seg < L.seg_end) return;
+            if (L.seg < L.seg_end) return rows;
         }
         L.ti += gridDim.x;
         enter_tile();
+        return rows;
     };
 
+    // K rows of the stages in flight, the oldest first.  Every thread walks the same cursor, so
+    // each keeps them in registers (a shared word would need a barrier between the prologue's
+    // write and the first step's read).
+    uint32_t held[STAGES];
     enter_tile();
 #pragma unroll
     for (int s = 0; s < STAGES - 1; ++s) {
-        issue(s);
+        held[s] = issue(s);
         cp_async_commit();
     }
 
@@ -307,8 +313,10 @@ __global__ void __launch_bounds__(NTHREADS, MINB) gemm_f64_grouped(const DevProb
         const uint32_t M = pr.M, N = pr.N;
         const bool inside = tl.m0 + wm < M && tl.n0 + wn < N;  // any of this warp's tile
         for (uint32_t st = 0; st < tl.nsteps; ++st) {
-            const uint32_t kn = st_k[slot];  // written when the stage was issued, a barrier ago
-            issue((slot + STAGES - 1) % STAGES);
+            const uint32_t kn = held[0];
+            held[STAGES - 1] = issue((slot + STAGES - 1) % STAGES);
+#pragma unroll
+            for (int s = 0; s < STAGES - 1; ++s) held[s] = held[s + 1];
             cp_async_commit();
             cp_async_wait<STAGES - 1>();
             __syncthreads();
