@@ -12,7 +12,7 @@
 // the CTAs exchange are the inner products: each CTA publishes its partial sums, every CTA
 // waits for all of them and adds them in the same order, so all hold the same coefficients
 // without a second exchange, and a solve is bitwise reproducible.  What bounds it are those
-// exchanges (iteration k has k + 4 of them, 2k + 5 with refinement) and the chain of
+// exchanges (k + 4 of them with k + 1 basis vectors, 2k + 6 with refinement) and the chain of
 // rotations of the k x k eigenproblem, which every CTA solves for itself; as separate
 // launches, one per inner product and vector operation (about 30 per iteration), it was
 // the launches and their drains.
@@ -361,8 +361,10 @@ __device__ void ritz(StepShared& sh, int k) {
                 sh.cs[lane][0] = c;
                 sh.cs[lane][1] = s;
             }
-            if (!__any_sync(0xffffffffu, any)) continue;
+            // the vote orders no memory: without it a lane that sums A at the next sweep could miss a
+            // dropped pair that another lane cleared
             __syncwarp();
+            if (!__any_sync(0xffffffffu, any)) continue;
             // A <- A J and Z <- Z J, then A <- J^T A: one row (column) of one pair per lane at a
             // time, so that the lanes' reads do not wait for each other's writes
             for (int e = lane; e < np * k; e += 32) {

@@ -95,3 +95,46 @@ def test_graph_solver_reused_and_reproducible():
     xo = torch.zeros_like(xd)
     theta, st = plan.solve(xd.data_ptr(), xo.data_ptr(), xd.numel(), tol=1e-10, max_iter=8)
     assert abs(theta - outs[0][0]) <= 1e-12 * abs(theta) and st.iterations == outs[0][2]
+
+
+def test_both_solvers_repeat_bitwise_on_staged_plans():
+    """At a size where H·psi runs its GEMM stages (blocks of up to 36 rows): twenty solves per
+    mode give one energy and one vector each, and the modes agree to 1e-12."""
+    ch, plan, keep, x0, rng = _setup("hubbard", 14, 6, seed=12, m=600)
+    xd = E.to_device(x0)
+    energy = []
+    for mode in MODES:
+        plan.set_solver(mode)
+        first = None
+        for _ in range(20):
+            xo = torch.zeros_like(xd)
+            theta, st = plan.solve(xd.data_ptr(), xo.data_ptr(), xd.numel(), tol=0.0, max_iter=6)
+            assert st.iterations == 6
+            got = (theta, xo.cpu().numpy())
+            first = first or got
+            assert got[0] == first[0] and np.array_equal(got[1], first[1])
+        energy.append(first[0])
+    assert abs(energy[0] - energy[1]) <= 1e-12 * abs(energy[1])
+
+
+def test_solve_continued_from_its_own_result():
+    """From an almost converged vector the projected matrix is diagonal but for entries that the
+    eigenproblem drops against the diagonal (whole wavefronts without a rotation): energy and
+    residual are the oracle's, and twenty solves give one bit pattern."""
+    ch, plan, keep, x0, rng = _setup("hubbard", 12, 5, seed=33, m=48)
+    xd = E.to_device(x0)
+    xo = torch.zeros_like(xd)
+    for _ in range(3):
+        plan.solve(xd.data_ptr(), xo.data_ptr(), xd.numel(), tol=1e-9, max_iter=32)
+        xd.copy_(xo)
+    x1 = xd.cpu().numpy()
+    theta_ref, _, it_ref, _, r_ref = JD.jcd(ch.hpsi, x1, tol=1e-11, max_iter=4)
+    first = None
+    for _ in range(20):
+        theta, st = plan.solve(xd.data_ptr(), xo.data_ptr(), xd.numel(), tol=1e-11, max_iter=4)
+        got = (theta, xo.cpu().numpy())
+        first = first or got
+        assert got[0] == first[0] and np.array_equal(got[1], first[1])
+        assert st.iterations == it_ref and abs(theta - theta_ref) <= 1e-12 * abs(theta_ref)
+        # the residual is the difference of vectors of norm |theta|: a few roundings of theta
+        assert abs(st.residual - r_ref) <= 1e-8 * r_ref + 1e-13 * abs(theta_ref)
