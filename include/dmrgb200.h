@@ -171,6 +171,20 @@ dmrgb200_status dmrgb200_plan_destroy(dmrgb200_plan_t plan);
  * DMRGB200_INVALID_PLAN with a message for inconsistent input. */
 dmrgb200_status dmrgb200_plan_validate(const dmrgb200_plan_desc* desc);
 
+/* How the FP64 entry points would run a plan description (host only, no device needed): which
+ * form it is lowered to, a function of the description alone. */
+typedef struct {
+    uint32_t chained;      /* 1: chained products, one launch; 0: the three stages */
+    uint32_t chain_tiles;  /* output tiles of the chained form */
+    uint32_t chain_warps;  /* warps per tile there (0: not chained) */
+    uint32_t stage3_parts; /* K parts of the output block cut into most; 1: none is cut */
+    uint32_t stage3_zero_blocks; /* output blocks no cohort writes, which stage 3 sets to zero */
+    uint32_t reserved;
+    uint64_t stage1_steps; /* K steps of stage 1 on 32 x 64 tiles */
+    uint64_t stage1_steps_whole; /* the same with every T block formed, read or not */
+} dmrgb200_lowering;
+dmrgb200_status dmrgb200_plan_lowering(const dmrgb200_plan_desc* desc, dmrgb200_lowering* out);
+
 /* Batched H·psi (independent site problems in one plan): n H·psi plan
  * descriptions with their left / right boundary views are concatenated so that
  * each stage of dmrgb200_hpsi is one launch over the tiles of all instances.

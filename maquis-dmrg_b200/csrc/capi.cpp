@@ -595,6 +595,20 @@ dmrgb200_status dmrgb200_plan_validate(const dmrgb200_plan_desc* d) {
     DMRGB200_CATCH
 }
 
+dmrgb200_status dmrgb200_plan_lowering(const dmrgb200_plan_desc* d, dmrgb200_lowering* out) {
+    DMRGB200_TRY
+    if (!out) return fail(DMRGB200_INVALID_ARGUMENT, "null output");
+    dmrgb200_status st = dmrgb200_plan_validate(d);
+    if (st != DMRGB200_OK) return st;
+    FlatPlan f;
+    desc_to_flat(d, f);
+    const ProgramForm pf = program_form(f);
+    *out = dmrgb200_lowering{uint32_t(pf.chained),  pf.chain_tiles, pf.chain_warps,  pf.stage3_parts,
+                             pf.stage3_zero_blocks, 0,              pf.stage1_steps, pf.stage1_steps_whole};
+    return DMRGB200_OK;
+    DMRGB200_CATCH
+}
+
 dmrgb200_status dmrgb200_plan_create_batched(dmrgb200_context_t ctx, uint32_t n, const dmrgb200_plan_desc* descs,
                                              const dmrgb200_boundary_view* lefts,
                                              const dmrgb200_boundary_view* rights, uint64_t* in_base,

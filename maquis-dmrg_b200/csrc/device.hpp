@@ -288,6 +288,15 @@ void build_alpha_dm(FlatPlan const& p, std::vector<uint64_t> const& dm, GemmList
 cudaError_t scale_buffer(double* x, uint64_t n, double a, cudaStream_t st);
 
 // ---- lowering helpers shared by the forward and adjoint programs ----
+// How the general entry points would run a plan (host work only)
+struct ProgramForm {
+    bool chained = false;
+    uint32_t chain_tiles = 0, chain_warps = 0;
+    uint32_t stage3_parts = 1, stage3_zero_blocks = 0;
+    uint64_t stage1_steps = 0, stage1_steps_whole = 0;
+};
+ProgramForm program_form(FlatPlan const& p);
+
 DevOp dev_op(uint16_t buf, uint64_t off, uint32_t ld, bool trans, uint64_t bstride = 0);
 void gemm_add_tiles(GemmList& gl, uint32_t prob, uint32_t nbatch);
 void gemm_sort_tiles(GemmList& gl);

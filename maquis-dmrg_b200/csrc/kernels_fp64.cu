@@ -1041,8 +1041,9 @@ bool split_list(GemmList const& gl, uint32_t target, GemmList& out) {
         DevProb pr = gl.probs[i];
         uint64_t steps = 0;
         for (uint32_t s = pr.seg_begin; s < pr.seg_end; ++s) steps += (gl.segs[s].K + 15) / 16;
+        // one part at least: a problem without segments stores zeros
         const uint32_t parts = nbatch[i] == 1 && pr.rows == DevProb::NO_ROWS && pr.M && pr.N
-                                   ? uint32_t(std::min<uint64_t>((steps + target - 1) / target, 16))
+                                   ? uint32_t(std::max<uint64_t>(1, std::min<uint64_t>((steps + target - 1) / target, 16)))
                                    : 1;
         uint32_t sg = pr.seg_begin, koff = 0;  // next segment and the K rows of it already given out
         uint64_t given = 0;
@@ -1092,6 +1093,40 @@ bool split_list(GemmList const& gl, uint32_t target, GemmList& out) {
     return true;
 }
 }  // namespace
+
+ProgramForm program_form(FlatPlan const& p) {
+    // any addresses do: nothing is read
+    auto ptrs = [](std::vector<uint32_t> const& ci) {
+        uint32_t n = 0;
+        for (uint32_t c : ci) n = std::max(n, c + 1);
+        return std::vector<uint64_t>(n, 8);
+    };
+    const bool hpsi = p.kind == KIND_HPSI;
+    const std::vector<uint64_t> s1 = ptrs(p.t_ci), s3 = hpsi ? ptrs(p.c_ci) : std::vector<uint64_t>(),
+                                out = hpsi ? std::vector<uint64_t>() : ptrs(p.c_out_ci);
+    DeviceProgram prog;
+    compile_program(p, s3, s1, out, prog, true, true);
+    ProgramForm f;
+    f.chained = prog.chained;
+    f.chain_tiles = uint32_t(prog.chain.tiles.size());
+    f.chain_warps = prog.chained ? uint32_t(prog.chain.split) : 0;
+    GemmList const& g3 = prog.own3 ? prog.stage3f : prog.stage3;
+    for (auto const& s : prog.stage3f.splits) f.stage3_parts = std::max(f.stage3_parts, s.parts);
+    for (auto const& pr : g3.probs)
+        if (pr.seg_begin == pr.seg_end && pr.M && pr.N) ++f.stage3_zero_blocks;
+    auto steps = [](GemmList const& gl) {
+        uint64_t n = 0;
+        for (auto const& t : gl.tiles) n += t.nsteps;
+        return n;
+    };
+    f.stage1_steps = f.stage1_steps_whole = steps(prog.stage1);
+    if (p.kind != KIND_LEFT && p.n_t()) {
+        GemmList whole;
+        stack_stage1(p, s1, t_offsets(p, nullptr), whole);
+        f.stage1_steps_whole = steps(whole);
+    }
+    return f;
+}
 
 void compile_program(FlatPlan const& p, std::vector<uint64_t> const& stage3_bnd,
                      std::vector<uint64_t> const& stage1_bnd, std::vector<uint64_t> const& outptr,

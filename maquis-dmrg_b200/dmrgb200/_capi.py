@@ -101,6 +101,13 @@ class BlockCopy(C.Structure):
 SCALE_NONE, SCALE_ROWS, SCALE_COLS = 0, 1, 2
 
 
+class Lowering(C.Structure):
+    """dmrgb200_lowering: the form a plan runs in."""
+    _fields_ = [("chained", C.c_uint32), ("chain_tiles", C.c_uint32), ("chain_warps", C.c_uint32),
+                ("stage3_parts", C.c_uint32), ("stage3_zero_blocks", C.c_uint32), ("reserved", C.c_uint32),
+                ("stage1_steps", C.c_uint64), ("stage1_steps_whole", C.c_uint64)]
+
+
 vp = C.c_void_p
 _sigs = {
     "dmrgb200_status_string": ([C.c_int], C.c_char_p),
@@ -123,6 +130,7 @@ _sigs = {
     "dmrgb200_plan_create_batched": ([vp, C.c_uint32, C.POINTER(PlanDesc), C.POINTER(BoundaryView),
                                       C.POINTER(BoundaryView), u64p, u64p, C.POINTER(vp)], C.c_int),
     "dmrgb200_plan_validate": ([C.POINTER(PlanDesc)], C.c_int),
+    "dmrgb200_plan_lowering": ([C.POINTER(PlanDesc), C.POINTER(Lowering)], C.c_int),
     "dmrgb200_calibrate": ([C.c_int, f64p], C.c_int),
     "dmrgb200_plan_flops": ([vp, u64p], C.c_int),
     "dmrgb200_plan_scratch_bytes": ([vp, u64p], C.c_int),

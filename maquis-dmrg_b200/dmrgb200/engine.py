@@ -191,6 +191,15 @@ class Context:
             self.handle = None
 
 
+def lowering(plan: dict) -> capi.Lowering:
+    """The form the device library would run a plan in (dmrgb200_plan_lowering; host only)."""
+    desc, keep = capi.numpy_to_desc(plan)
+    out = capi.Lowering()
+    capi.check(capi.lib.dmrgb200_plan_lowering(C.byref(desc), C.byref(out)), "plan_lowering")
+    del keep
+    return out
+
+
 class DevicePlan:
     """A plan bound to device boundaries (dmrgb200_plan_create)."""
 

@@ -139,3 +139,32 @@ def test_split_stage3_matches_oracle(L, m):
     plan.hpsi(xd.data_ptr(), yd.data_ptr())
     torch.cuda.synchronize()
     assert np.array_equal(yd.cpu().numpy(), y)  # parts are added in order, whichever arrives last
+
+
+@pytest.mark.parametrize("L,m,drop", [(10, 150, 3), (8, 60, 2)])
+def test_blocks_without_a_cohort_are_zero(L, m, drop):
+    """Output blocks that no cohort writes come out as zeros, not as what y held, with stage 3
+    cut into K parts and not, from device and from host buffers."""
+    ctx = E.Context(0)
+    model = SU.quantum_chemistry(L, L, 0)
+    bonds = [list(b) for b in SU.synthetic_bonds(L, model.total_charge, m)]
+    bonds[L // 2 - 2] = bonds[L // 2 - 2][drop:]
+    rng = np.random.default_rng(4)
+    ch = OracleChain(model, bonds, S.random_mps(SU.PHYS, bonds, rng), L // 2 - 1)
+    p = ch.sched.plan
+    assert len(set(p["c_rb"].tolist())) < len(p["out_rows"])
+    plan, keep = _plan(ctx, ch)
+    x = rng.standard_normal(int(p["in_size"]))
+    ref = ch.hpsi(x)
+    mask = np.zeros(len(ref), bool)
+    for r, c, o in zip(p["out_rows"], p["out_cols"], p["out_off"]):
+        mask[int(o):int(o) + int(r) * int(c)] = True
+    xd = E.to_device(x)
+    yd = torch.full((len(ref),), np.nan, dtype=torch.float64, device="cuda")
+    xh, yh = torch.from_numpy(x.copy()).pin_memory(), torch.full((len(ref),), np.nan, dtype=torch.float64).pin_memory()
+    plan.hpsi(xd.data_ptr(), yd.data_ptr())
+    plan.hpsi_host(xh.data_ptr(), yh.data_ptr())
+    torch.cuda.synchronize()
+    for y in (yd.cpu().numpy(), yh.numpy()):
+        assert _rel(y[mask], ref[mask]) <= 1e-12
+        assert np.all(y[mask][ref[mask] == 0.0] == 0.0)
