@@ -788,10 +788,14 @@ std::vector<std::vector<char>> t_blocks_read(FlatPlan const& p) {
 // row-table problem: A row r is row r' of task t's psi slice, C row r is row r'
 // of T_t (leading dimension = the task's row count), so one tile covers several
 // small psi blocks instead of padding each to a full tile.  T blocks that no term reads
-// are left out where that saves a tenth of a cohort's blocks or more: the tasks are then
-// stacked by the set of blocks they need, one problem per run of adjacent blocks.  (In
-// quantum chemistry nearly all blocks are read, by slightly different sets per task:
-// splitting there would undo the stacking for a percent of the work.)
+// can be left out: the tasks are then stacked by the set of blocks they need, one problem
+// per run of adjacent blocks (a run goes on over a gap where that takes no more tiles).  That
+// undoes some of the stacking, so a cohort is cut up only where it saves a tenth of its tile
+// K steps or more, on tiles of 32 rows and of 64 (the shapes of most variants).  Lattice
+// chains save 19 to 34% (Hubbard L = 64, m = 1024, middle: 7352 steps to 5072, H psi 57.8 us to 52.4;
+// Heisenberg m = 1024 84.5 to 77.4).  Quantum chemistry reads nearly all blocks at the middle
+// and, left of it, slightly different sets per task: cut up by the share of blocks saved, L =
+// 12, m = 300, sites 3 and 4 would go from 3017 and 13260 steps to 9693 and 22089.
 void stack_stage1(FlatPlan const& p, std::vector<uint64_t> const& stage1_bnd, std::vector<uint64_t> const& t_off,
                   GemmList& g1, std::vector<char> const* keep = nullptr, bool skip_unread = false) {
     g1 = GemmList();
@@ -836,24 +840,56 @@ void stack_stage1(FlatPlan const& p, std::vector<uint64_t> const& stage1_bnd, st
         g1.probs.push_back(pr);
         add_tiles(g1, uint32_t(g1.probs.size() - 1), nbatch);
     };
+    // K steps of one problem of M stacked rows and nb blocks on tiles of bm x 64
+    auto steps = [&](uint32_t t0, uint64_t bm, uint64_t M, uint64_t nb) {
+        const uint64_t Nf = p.t_bcols[t0], nt = p.t_trans[t0] ? nb * ((Nf + 63) / 64) : (nb * Nf + 63) / 64;
+        return (M + bm - 1) / bm * nt * ((p.t_brows[t0] + 15) / 16);
+    };
+    struct Piece {
+        std::vector<uint32_t> const* tasks;
+        uint32_t b0, nb;
+    };
     for (auto const& kv : groups) {
-        const uint32_t nb = p.t_nb[kv.second.front()];
-        uint64_t used = 0;
-        if (skip_unread)
-            for (uint32_t t : kv.second) used += uint64_t(std::count(read[t].begin(), read[t].end(), 1));
-        if (!skip_unread || used * 10 > uint64_t(nb) * kv.second.size() * 9) {
+        const uint32_t t0 = kv.second.front(), nb = p.t_nb[t0];
+        if (!skip_unread) {
             problem(kv.second, 0, nb);
             continue;
         }
         std::map<std::vector<char>, std::vector<uint32_t>> by_set;
         for (uint32_t t : kv.second) by_set[read[t]].push_back(t);
-        for (auto const& sv : by_set)
+        auto rows = [&](std::vector<uint32_t> const& tasks) {
+            uint64_t M = 0;
+            for (uint32_t t : tasks) M += p.in_rows[p.t_lb[t]];
+            return M;
+        };
+        std::vector<Piece> pieces;
+        uint64_t c32 = 0, c64 = 0;
+        for (auto const& sv : by_set) {
+            const uint64_t M = rows(sv.second);
             for (uint32_t b = 0; b < nb;) {
                 uint32_t e = b;
                 while (e < nb && sv.first[e]) ++e;
-                if (e > b) problem(sv.second, b, e - b);
+                if (e > b) {
+                    // over a gap to the run before, where the wider problem has no more tiles
+                    if (!pieces.empty() && pieces.back().tasks == &sv.second &&
+                        steps(t0, 32, M, e - pieces.back().b0) <= steps(t0, 32, M, pieces.back().nb) + steps(t0, 32, M, e - b))
+                        pieces.back().nb = e - pieces.back().b0;
+                    else
+                        pieces.push_back({&sv.second, b, e - b});
+                }
                 b = e + 1;
             }
+        }
+        for (auto const& x : pieces) {
+            c32 += steps(t0, 32, rows(*x.tasks), x.nb);
+            c64 += steps(t0, 64, rows(*x.tasks), x.nb);
+        }
+        const uint64_t M = rows(kv.second);
+        if (10 * c32 > 9 * steps(t0, 32, M, nb) || 10 * c64 > 9 * steps(t0, 64, M, nb)) {
+            problem(kv.second, 0, nb);
+            continue;
+        }
+        for (auto const& x : pieces) problem(*x.tasks, x.b0, x.nb);
     }
     sort_tiles(g1);
 }

@@ -48,3 +48,24 @@ def test_blocks_without_a_cohort_stay_in_stage3(L, m, i, drop, cut):
     empty = len(plan["out_rows"]) - len(set(plan["c_rb"].tolist()))
     assert (empty > 0) == (drop > 1)
     assert form.stage3_zero_blocks == empty
+
+
+@pytest.mark.parametrize("L,m,sites", [(12, 300, range(1, 10)), (16, 512, (2, 3, 4, 5, 6, 7, 9))])
+def test_quantum_chemistry_stage1_keeps_its_stacked_rows(L, m, sites):
+    """Leaving out T blocks that no term reads never costs tile steps: left of the middle each
+    task reads a set of its own, and problems by set would undo the row stacking."""
+    model = SU.quantum_chemistry(L, L, 0)
+    bonds = SU.synthetic_bonds(L, model.total_charge, m)
+    for i in sites:
+        form = E.lowering(hpsi_plan(model, bonds, i))
+        assert 0 < form.stage1_steps <= form.stage1_steps_whole, i
+
+
+@pytest.mark.parametrize("model,width,m,i,share", [(M.fermi_hubbard(64), 3.5, 1024, 31, 0.70), (M.fermi_hubbard(64), 3.5, 1600, 10, 0.70),
+                                                   (M.heisenberg(32), 10.0, 1024, 15, 0.81)])
+def test_lattice_stage1_leaves_unread_blocks_out(model, width, m, i, share):
+    """On lattice chains a fifth to a third of the T blocks is read by no term."""
+    from dmrgb200 import mps as S
+    bonds = S.synthetic_bonds(model.phys, len(model.mpo), model.total_charge, m, width)
+    form = E.lowering(hpsi_plan(model, bonds, i))
+    assert not form.chained and form.stage1_steps <= share * form.stage1_steps_whole
