@@ -207,8 +207,10 @@ dmrgb200_status dmrgb200_plan_scratch_bytes(dmrgb200_plan_t plan, uint64_t* byte
 /* y = H_eff x for a DMRGB200_PLAN_HPSI plan.  x and y are device vectors laid
  * out as the plan's in/out blocks (DavidsonVector layout,
  * davidson_vector.cpp:87-152); y's block elements are overwritten, its padding
- * is left untouched.  Replaces super_hamil_mv (super_hamil_mv.hpp:100-155) and
- * ietl::mult (ietl_interface_dv.h:112-118).  DMRGB200_PREC_FP64_EMULATED runs
+ * is left untouched.  y may be x or overlap it or the right boundary's blocks: the
+ * plan then runs its stages, which have read both before they write y, also where it
+ * would run as chained products.  Replaces super_hamil_mv (super_hamil_mv.hpp:100-155)
+ * and ietl::mult (ietl_interface_dv.h:112-118).  DMRGB200_PREC_FP64_EMULATED runs
  * the T and cohort contractions on the INT8 tensor cores (Ozaki split, see
  * dmrgb200_plan_set_slices) and the S build in FP64, stream-ordered like the
  * FP64 path.  The first emulated call of a plan allocates its digit-plane
@@ -478,7 +480,8 @@ dmrgb200_status dmrgb200_hpsi_noalloc(const dmrgb200_plan_desc* desc, const dmrg
  * (plan in-blocks); bra: left-paired (left step) or right-paired (right step)
  * device tensor (plan out-blocks); out: device pointers of the new boundary's
  * cohorts (indexed by c_out_ci); every stored element of those cohorts is
- * written.
+ * written.  The new cohorts may overlap the ket or the input boundary (not the bra), which
+ * are read before anything is written.
  * Replaces the GPU branches of overlap_mpo_left_step / overlap_mpo_right_step
  * (move_boundary.hpp:215-259, :342-384). */
 dmrgb200_status dmrgb200_step_execute(dmrgb200_plan_t plan, const double* ket, const double* bra,

@@ -50,6 +50,37 @@ struct dmrgb200_schedule_s {
     FlatPlan flat;
 };
 
+// Address ranges [first, second), for the overlap of a call's inputs and outputs
+struct Ranges {
+    std::vector<std::pair<uint64_t, uint64_t>> r;  // sorted, disjoint after close()
+    void add(uint64_t at, uint64_t elems) {
+        if (elems) r.emplace_back(at, at + 8 * elems);
+    }
+    void close() {
+        std::sort(r.begin(), r.end());
+        size_t n = 0;
+        for (auto const& x : r) {
+            if (n && x.first <= r[n - 1].second) r[n - 1].second = std::max(r[n - 1].second, x.second);
+            else r[n++] = x;
+        }
+        r.resize(n);
+    }
+    bool meets(uint64_t at, uint64_t elems) const {
+        const uint64_t end = at + 8 * elems;
+        auto it = std::upper_bound(r.begin(), r.end(), std::make_pair(at, ~uint64_t(0)));
+        if (it != r.begin() && std::prev(it)->second > at && elems) return true;
+        return elems && it != r.end() && it->first < end;
+    }
+};
+// the boundary blocks that the T tasks of a plan read
+Ranges t_reads(FlatPlan const& f, std::vector<uint64_t> const& bnd) {
+    Ranges g;
+    for (uint32_t t = 0; t < f.n_t(); ++t)
+        g.add(bnd[f.t_ci[t]], uint64_t(f.t_nb[t]) * f.t_brows[t] * f.t_bcols[t]);
+    g.close();
+    return g;
+}
+
 struct dmrgb200_plan_s {
     FlatPlan flat;
     DeviceProgram prog;
@@ -57,6 +88,11 @@ struct dmrgb200_plan_s {
     double* T = nullptr;
     double* S = nullptr;
     std::vector<uint64_t> stage1_bnd, stage3_bnd;
+    // Chained products read x (ket) and the T tasks' boundary while other CTAs write the
+    // output; the stages have read both by then.  So calls whose output overlaps one of them run
+    // the stages: the boundary blocks read, and of a step the output blocks and whether the two meet.
+    Ranges reads, step_writes;
+    bool step_in_place = false;
     int device = 0;
     // per-stage timing
     bool timing = false;
@@ -265,6 +301,7 @@ dmrgb200_status finish_plan(std::unique_ptr<dmrgb200_plan_s>& p, dmrgb200_plan_t
     err = check_bound(p->flat, p->stage1_bnd, p->stage3_bnd);
     if (!err.empty()) return fail(DMRGB200_INVALID_PLAN, err);
     cudaGetDevice(&p->device);
+    p->reads = t_reads(p->flat, p->stage1_bnd);
     if (p->flat.kind == KIND_HPSI) {
         compile_program(p->flat, p->stage3_bnd, p->stage1_bnd, {}, p->prog, true, true);
         cudaError_t e = upload_program(p->prog);
@@ -298,6 +335,9 @@ dmrgb200_status run_step(dmrgb200_plan_s* p, const double* ket, const double* br
         if (p->flat.c_out_ci[c] >= outp.size() || !outp[p->flat.c_out_ci[c]])
             return fail(DMRGB200_INVALID_ARGUMENT, "output boundary view misses a cohort");
     cudaError_t e;
+    auto overlaps = [&] {
+        return p->step_in_place || p->step_writes.meets(reinterpret_cast<uint64_t>(ket), p->flat.in_size);
+    };
     if (!p->step_valid || p->step_outp != outp) {
         p->drop_step();
         compile_program(p->flat, {}, p->stage1_bnd, outp, p->step_prog, true, true);
@@ -307,6 +347,15 @@ dmrgb200_status run_step(dmrgb200_plan_s* p, const double* ket, const double* br
         }
         p->step_valid = true;
         p->step_outp = outp;
+        p->step_writes = Ranges();
+        p->step_in_place = false;
+        for (uint32_t c = 0; c < p->flat.n_cohorts(); ++c) {
+            const uint64_t at = outp[p->flat.c_out_ci[c]],
+                           n = uint64_t(p->flat.c_ls[c]) * p->flat.c_rs[c] * p->flat.c_nsrows[c];
+            p->step_writes.add(at, n);
+            p->step_in_place = p->step_in_place || p->reads.meets(at, n);
+        }
+        p->step_writes.close();
         if (p->step_prog.t_elems && (e = cudaMalloc(&p->step_T, p->step_prog.t_elems * sizeof(double))) != cudaSuccess) {
             p->drop_step();
             return cuda_fail(e, "step T scratch");
@@ -319,7 +368,9 @@ dmrgb200_status run_step(dmrgb200_plan_s* p, const double* ket, const double* br
             const char* v = std::getenv("DMRGB200_AUTOTUNE");
             return !(v && v[0] == '0');
         }();
-        if (tune && !p->step_prog.chained && p->flat.flops() >= 50000000ull && !capturing(stream)) {
+        // (tuning writes the outputs before the step has read its inputs)
+        const bool over = overlaps();
+        if (tune && !p->step_prog.chained && !over && p->flat.flops() >= 50000000ull && !capturing(stream)) {
             // the variants run the whole step (outputs included): the run below rewrites them
             if ((e = tune_program(p->step_prog, reinterpret_cast<uint64_t>(ket), reinterpret_cast<uint64_t>(bra),
                                   p->step_T, p->step_S, stream)) != cudaSuccess) {
@@ -329,7 +380,7 @@ dmrgb200_status run_step(dmrgb200_plan_s* p, const double* ket, const double* br
         }
     }
     e = run_program(p->step_prog, reinterpret_cast<uint64_t>(ket), reinterpret_cast<uint64_t>(bra), p->step_T,
-                    p->step_S, stream, p->timing ? p->ev : nullptr);
+                    p->step_S, stream, p->timing ? p->ev : nullptr, p->step_prog.chained && overlaps());
     // the wait-timeout word comes back with the step's own synchronisation
     const bool word = p->step_prog.d_err != nullptr;
     if (word && !p->step_err && cudaHostAlloc(&p->step_err, sizeof(int), cudaHostAllocDefault) != cudaSuccess)
@@ -689,12 +740,15 @@ dmrgb200_status dmrgb200_hpsi(dmrgb200_plan_t plan, const double* x, double* y, 
     if (prec == DMRGB200_PREC_FP64_EMULATED) return hpsi_emulated(plan, x, y, static_cast<cudaStream_t>(cuda_stream));
     if (prec != DMRGB200_PREC_FP64) return fail(DMRGB200_INVALID_ARGUMENT, "unknown precision");
     if (plan->timing) plan->collect();
-    {
+    const uint64_t xa = reinterpret_cast<uint64_t>(x), ya = reinterpret_cast<uint64_t>(y), nx = plan->flat.in_size,
+                   ny = plan->flat.out_size;
+    const bool over = (xa < ya + 8 * ny && ya < xa + 8 * nx) || plan->reads.meets(ya, ny);
+    if (!over) {  // (tuning writes y before H psi has read its inputs)
         cudaError_t te = plan_ensure_tuned(plan, x, y, static_cast<cudaStream_t>(cuda_stream));
         if (te != cudaSuccess) return cuda_fail(te, "grouped GEMM autotuning");
     }
-    cudaError_t e = run_program(plan->prog, reinterpret_cast<uint64_t>(x), reinterpret_cast<uint64_t>(y), plan->T,
-                                plan->S, static_cast<cudaStream_t>(cuda_stream), plan->timing ? plan->ev : nullptr);
+    cudaError_t e = run_program(plan->prog, xa, ya, plan->T, plan->S, static_cast<cudaStream_t>(cuda_stream),
+                                plan->timing ? plan->ev : nullptr, over);
     if (e != cudaSuccess) return cuda_fail(e, "hpsi launch");
     if (plan->timing) plan->pending = true;
     return DMRGB200_OK;

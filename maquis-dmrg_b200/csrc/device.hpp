@@ -271,8 +271,9 @@ void free_program(DeviceProgram& prog);
 
 // Launch the three stages on a stream; T and S are the scratch buffers.
 // ev (optional): four events recorded before stage 1 and after stages 1, 2, 3.
+// staged: the stages also where the plan runs as chained products.
 cudaError_t run_program(DeviceProgram const& prog, uint64_t in, uint64_t out, double* T, double* S,
-                        cudaStream_t stream, cudaEvent_t const* ev = nullptr);
+                        cudaStream_t stream, cudaEvent_t const* ev = nullptr, bool staged = false);
 
 int device_sm_count();
 // stages 1 and 2 only (T and the S build), as run_program launches them

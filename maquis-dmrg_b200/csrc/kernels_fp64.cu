@@ -1914,7 +1914,7 @@ cudaError_t run_stages12(DeviceProgram const& prog, uint64_t in, uint64_t out, d
 }
 
 cudaError_t run_program(DeviceProgram const& prog, uint64_t in, uint64_t out, double* T, double* S,
-                        cudaStream_t stream, cudaEvent_t const* ev) {
+                        cudaStream_t stream, cudaEvent_t const* ev, bool staged) {
     Bases bs{};
     bs.b[BUF_IN] = in;
     bs.b[BUF_OUT] = out;
@@ -1922,7 +1922,7 @@ cudaError_t run_program(DeviceProgram const& prog, uint64_t in, uint64_t out, do
     bs.b[BUF_S] = reinterpret_cast<uint64_t>(S);
     bs.b[BUF_ABS] = 0;
     if (ev) cudaEventRecord(ev[0], stream);
-    if (prog.chained) {
+    if (prog.chained && !staged) {
         // timed as the contraction (stage 2)
         if (ev) cudaEventRecord(ev[1], stream);
         if (ev) cudaEventRecord(ev[2], stream);

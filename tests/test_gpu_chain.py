@@ -168,3 +168,73 @@ def test_blocks_without_a_cohort_are_zero(L, m, drop):
     for y in (yd.cpu().numpy(), yh.numpy()):
         assert _rel(y[mask], ref[mask]) <= 1e-12
         assert np.all(y[mask][ref[mask] == 0.0] == 0.0)
+
+
+@pytest.mark.parametrize("name,L,m,i", [("heisenberg", 16, 64, 7), ("hubbard", 14, 333, 4)])
+def test_chained_hpsi_in_place(name, L, m, i):
+    """y = x, y overlapping x, and y over the right boundary's blocks: the oracle's H·psi, and
+    the bits of the stages (chained products would read what other CTAs have overwritten)."""
+    ctx = E.Context(0)
+    model, bonds, tensors, rng = make_chain(name, L, 0, seed=m, synthetic_m=m)
+    ch = OracleChain(model, bonds, tensors, i)
+    assert E.lowering(ch.sched.plan).chained
+    x = random_psi(ch.p12, ch.left, ch.right, rng).data
+    ref, n = ch.hpsi(x), len(x)
+    plan, keep = _plan(ctx, ch)
+    pinned, keep2 = _plan(ctx, ch)
+    pinned.set_gemm_variants(0, 0)
+    buf = torch.zeros(2 * n, dtype=torch.float64, device="cuda")
+    xd, staged = E.to_device(x), torch.zeros(n, dtype=torch.float64, device="cuda")
+    pinned.hpsi(xd.data_ptr(), staged.data_ptr())
+    for shift in (0, 0, 0, 0, 8, 128, n // 2):
+        buf[:n] = xd
+        buf[n:] = 0.0
+        plan.hpsi(buf.data_ptr(), buf[shift:].data_ptr())
+        torch.cuda.synchronize()
+        mask = torch.from_numpy(ref != 0.0).cuda()
+        assert _rel(buf[shift:shift + n][mask].cpu().numpy(), ref[ref != 0.0]) <= TOL, shift
+        assert torch.equal(buf[shift:shift + n][mask], staged[mask]), shift
+    # y at the start of the right boundary's storage (which it overwrites)
+    Lb = E.to_device(ch.Lval)
+    Rb = torch.zeros(max(len(ch.Rval), n), dtype=torch.float64, device="cuda")
+    Rb[:len(ch.Rval)] = E.to_device(ch.Rval)
+    over = E.DevicePlan(ctx, ch.sched.plan, left_addr=ch.Lidx.cohort_addresses(Lb.data_ptr()),
+                        other_addr=ch.Ridx.cohort_addresses(Rb.data_ptr()))
+    over.hpsi(xd.data_ptr(), Rb.data_ptr())
+    torch.cuda.synchronize()
+    assert torch.equal(Rb[:n][mask], staged[mask])
+
+
+@pytest.mark.parametrize("name,L,m", [("heisenberg", 16, 64), ("hubbard", 12, 333)])
+def test_chained_steps_in_place(name, L, m):
+    """New boundaries written over the old ones, and over the ket, from the ends to the middle."""
+    ctx = E.Context(0)
+    model, bonds, tensors, _ = make_chain(name, L, 0, seed=3, synthetic_m=m)
+    chained = 0
+    for left in (True, False):
+        idx = E.edge_bindex(model.symm, bonds[0] if left else bonds[L])
+        val = idx.edge_values()
+        for p in (range(L // 2) if left else range(L - 1, L // 2, -1)):
+            W, t = M.MPOHandle(model.mpo[p], model.symm), tensors[p]
+            if left:
+                sch, nidx = E.schedule_left_step(model.phys, bonds[p], bonds[p + 1], W, idx, True)
+                ref = O.left_step(sch.plan, val, idx, t.data, t.left_paired(), nidx)
+                bra = E.to_device(t.left_paired())
+            else:
+                sch, nidx = E.schedule_right_step(model.phys, bonds[p], bonds[p + 1], W, idx, True)
+                ref = O.right_step(sch.plan, val, idx, t.data, t.data, nidx)
+                bra = E.to_device(t.data)
+            chained += int(E.lowering(sch.plan).chained)
+            for over in ("boundary", "ket"):
+                old = torch.zeros(max(len(val), len(ref)), dtype=torch.float64, device="cuda")
+                old[:len(val)] = E.to_device(val)
+                ket = torch.zeros(max(len(t.data), len(ref)), dtype=torch.float64, device="cuda")
+                ket[:len(t.data)] = E.to_device(t.data)
+                addr = idx.cohort_addresses(old.data_ptr())
+                plan = E.DevicePlan(ctx, sch.plan, **({"left_addr": addr} if left else {"other_addr": addr}))
+                out = old if over == "boundary" else ket
+                plan.step(ket.data_ptr(), bra.data_ptr(), nidx.cohort_addresses(out.data_ptr()))
+                got = out.cpu().numpy()[:len(ref)]  # the gaps between cohorts keep what was there
+                assert _rel(got[ref != 0.0], ref[ref != 0.0]) <= TOL, (left, p, over)
+            idx, val = nidx, ref
+    assert chained >= L // 2
