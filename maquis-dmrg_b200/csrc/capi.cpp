@@ -116,7 +116,7 @@ struct dmrgb200_plan_s {
     // H psi with host buffers (built on first use): split program, device copies of x
     // and y, a copy stream and its events
     static constexpr uint32_t PIPE_PARTS = 4;
-    bool pipe_built = false;
+    bool pipe_ready = false;  // pipe holds a complete program; the buffers below have their own nulls
     PipelineProgram pipe;
     double* hx = nullptr;
     double* hy = nullptr;
@@ -183,6 +183,7 @@ dmrgb200_status fail(dmrgb200_status s, std::string const& msg) {
 }
 
 dmrgb200_status cuda_fail(cudaError_t e, const char* where) {
+    cudaGetLastError();  // reported here: not to a later call's check of its launches
     return fail(e == cudaErrorMemoryAllocation ? DMRGB200_OUT_OF_MEMORY : DMRGB200_DEVICE_ERROR,
                 std::string(where) + ": " + cudaGetErrorString(e));
 }
@@ -689,20 +690,25 @@ dmrgb200_status dmrgb200_plan_create_batched(dmrgb200_context_t ctx, uint32_t n,
     DMRGB200_CATCH
 }
 
+static void drop_pipe_graph(dmrgb200_plan_t plan) {
+    if (plan->pipe_exec) cudaGraphExecDestroy(plan->pipe_exec);
+    plan->pipe_exec = nullptr;
+    plan->pipe_x = nullptr;
+    plan->pipe_y = nullptr;
+}
+
 dmrgb200_status dmrgb200_plan_destroy(dmrgb200_plan_t plan) {
     if (!plan) return DMRGB200_OK;
     if (plan->compiled) free_program(plan->prog);
     if (plan->adj_built) free_adjoint(plan->adj);
-    if (plan->pipe_built) {
-        free_pipeline(plan->pipe);
-        cudaFree(plan->hx);
-        cudaFree(plan->hy);
-        if (plan->pipe_exec) cudaGraphExecDestroy(plan->pipe_exec);
-        for (auto& e : plan->pev)
-            if (e) cudaEventDestroy(e);
-        if (plan->copy_stream) cudaStreamDestroy(plan->copy_stream);
-        if (plan->capture_stream) cudaStreamDestroy(plan->capture_stream);
-    }
+    free_pipeline(plan->pipe);
+    cudaFree(plan->hx);
+    cudaFree(plan->hy);
+    drop_pipe_graph(plan);
+    for (auto& e : plan->pev)
+        if (e) cudaEventDestroy(e);
+    if (plan->copy_stream) cudaStreamDestroy(plan->copy_stream);
+    if (plan->capture_stream) cudaStreamDestroy(plan->capture_stream);
     jd_graph_free(plan->jd);
     blas_handle_free(plan->blas);
     plan->drop_step();
@@ -760,37 +766,45 @@ dmrgb200_status dmrgb200_hpsi_host(dmrgb200_plan_t plan, const double* x_host, d
     if (plan->flat.kind != KIND_HPSI || !plan->compiled) return fail(DMRGB200_INVALID_PLAN, "plan is not an H psi plan");
     cudaStream_t st = static_cast<cudaStream_t>(cuda_stream);
     cudaError_t e;
-    if (plan->pipe_built && plan->pipe.chained != plan->prog.chained) {
+    if (plan->pipe_ready && plan->pipe.chained != plan->prog.chained) {
         // pinned GEMM variants replaced the chained products: the ranges are lowered again
+        drop_pipe_graph(plan);
+        plan->pipe_ready = false;
+    }
+    // what an earlier call could not allocate is tried again
+    if (!plan->pipe_ready) {
         free_pipeline(plan->pipe);
         if ((e = compile_pipeline(plan->flat, plan->stage3_bnd, plan->stage1_bnd, plan->prog, plan->PIPE_PARTS,
-                                  plan->pipe)) != cudaSuccess)
+                                  plan->pipe)) != cudaSuccess) {
+            free_pipeline(plan->pipe);
             return cuda_fail(e, "host-buffer program");
+        }
+        plan->pipe_ready = true;
     }
-    if (!plan->pipe_built) {
-        plan->pipe_built = true;  // released by dmrgb200_plan_destroy, also after a failure here
-        if ((e = compile_pipeline(plan->flat, plan->stage3_bnd, plan->stage1_bnd, plan->prog, plan->PIPE_PARTS,
-                                  plan->pipe)) != cudaSuccess)
-            return cuda_fail(e, "host-buffer program");
-        const size_t nx = std::max<uint64_t>(plan->flat.in_size, 1), ny = std::max<uint64_t>(plan->flat.out_size, 1);
-        if ((e = cudaMalloc(&plan->hx, nx * sizeof(double))) != cudaSuccess ||
-            (e = cudaMalloc(&plan->hy, ny * sizeof(double))) != cudaSuccess ||
-            // H psi writes only block elements: the padding copied back stays zero
-            (e = cudaMemset(plan->hy, 0, ny * sizeof(double))) != cudaSuccess ||
-            (e = cudaStreamCreateWithFlags(&plan->copy_stream, cudaStreamNonBlocking)) != cudaSuccess ||
-            (e = cudaStreamCreateWithFlags(&plan->capture_stream, cudaStreamNonBlocking)) != cudaSuccess)
+    const size_t nx = std::max<uint64_t>(plan->flat.in_size, 1), ny = std::max<uint64_t>(plan->flat.out_size, 1);
+    if (!plan->hx && (e = cudaMalloc(&plan->hx, nx * sizeof(double))) != cudaSuccess)
+        return cuda_fail(e, "host-buffer scratch");
+    if (!plan->hy) {
+        double* hy = nullptr;
+        if ((e = cudaMalloc(&hy, ny * sizeof(double))) != cudaSuccess) return cuda_fail(e, "host-buffer scratch");
+        // H psi writes only block elements: the padding copied back stays zero
+        if ((e = cudaMemset(hy, 0, ny * sizeof(double))) != cudaSuccess) {
+            cudaFree(hy);
             return cuda_fail(e, "host-buffer scratch");
-        for (auto& ev : plan->pev)
-            if ((e = cudaEventCreateWithFlags(&ev, cudaEventDisableTiming)) != cudaSuccess)
-                return cuda_fail(e, "host-buffer events");
+        }
+        plan->hy = hy;
     }
-    if (!plan->hx || !plan->copy_stream) return fail(DMRGB200_DEVICE_ERROR, "host-buffer program unavailable");
+    for (cudaStream_t* s : {&plan->copy_stream, &plan->capture_stream})
+        if (!*s && (e = cudaStreamCreateWithFlags(s, cudaStreamNonBlocking)) != cudaSuccess)
+            return cuda_fail(e, "host-buffer streams");
+    for (auto& ev : plan->pev)
+        if (!ev && (e = cudaEventCreateWithFlags(&ev, cudaEventDisableTiming)) != cudaSuccess)
+            return cuda_fail(e, "host-buffer events");
     if ((e = plan_ensure_tuned(plan, plan->hx, plan->hy, st)) != cudaSuccess)
         return cuda_fail(e, "grouped GEMM autotuning");
     if (!plan->pipe_exec || plan->pipe_x != x_host || plan->pipe_y != y_host) {
         // (re)capture for these host buffers on the plan's own stream
-        if (plan->pipe_exec) cudaGraphExecDestroy(plan->pipe_exec);
-        plan->pipe_exec = nullptr;
+        drop_pipe_graph(plan);
         cudaGraph_t g = nullptr;
         cudaStream_t cs = plan->capture_stream;
         if ((e = cudaStreamBeginCapture(cs, cudaStreamCaptureModeThreadLocal)) != cudaSuccess)
@@ -850,10 +864,7 @@ dmrgb200_status dmrgb200_hpsi_adjoint(dmrgb200_plan_t plan, const double* w, con
 static void drop_variant_graphs(dmrgb200_plan_t plan) {
     jd_graph_free(plan->jd);
     plan->jd = nullptr;
-    if (plan->pipe_exec) cudaGraphExecDestroy(plan->pipe_exec);
-    plan->pipe_exec = nullptr;
-    plan->pipe_x = nullptr;
-    plan->pipe_y = nullptr;
+    drop_pipe_graph(plan);
 }
 
 dmrgb200_status dmrgb200_plan_autotune(dmrgb200_plan_t plan, const double* x, double* y, void* cuda_stream,
