@@ -10,7 +10,7 @@
 // svd_cluster: blocks of up to 256 x 256, one thread-block cluster per block, pivoted QR
 // then one-sided Jacobi on R^T with the columns in registers (see the kernel).
 //
-// block_svd_jacobi: larger blocks, and the blocks svd_cluster hands back (an exactly zero
+// block_svd_jacobi: larger blocks, and the blocks svd_cluster hands back (a vanishing
 // pivot, non-finite input); one CTA of 16 warps per block, one-sided (Hestenes) Jacobi.  The block is
 // taken as m x n columns with n = min(rows, cols) (the transpose when rows < cols).
 // Column pairs are orthogonalised in round-robin order, n/2 disjoint pairs per
@@ -227,8 +227,9 @@ __device__ __forceinline__ void cluster_sync(cooperative_groups::cluster_group c
 // CTA, up to 8 CTAs) and never leave the registers.  The 45 blocks (17 to 208 square) of a
 // split at m = 1024 with singular values over eight decades: 4.9 ms, against 90 ms by
 // block_svd_jacobi (one CTA per block, columns in L2, no pivoting).
-// A block with an exactly zero or non-finite pivot, or that does not converge, is handed
-// to block_svd_jacobi (general = 1), which keeps V orthonormal there.
+// A block with a zero, vanishing (below 1e-140 of the largest element) or non-finite pivot,
+// or that does not converge, is handed to block_svd_jacobi (general = 1), which keeps V
+// orthonormal there.
 template <int EPL>
 struct SvdShared {
     double col[SVD_WARPS][2][2][EPL * 32];  // [warp][round parity][L, J][element]
@@ -336,7 +337,9 @@ __global__ void __launch_bounds__(SVD_THREADS) svd_cluster(SvdBlock* blocks) {
                 bid = id;
             }
         }
-        ok = best > 0.0 && best < 1.7976931348623157e308;
+        // (a squared norm near the subnormal range has lost digits, and a reflector made from it
+        // is not orthogonal: such columns, 1e-140 of the largest element, are handed over too)
+        ok = best > 1e-280 && best < 1.7976931348623157e308;
         if (!ok) break;
         if (active && (bid == idx || bid == idy)) {
             const bool first = bid == idx;

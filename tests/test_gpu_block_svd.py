@@ -131,6 +131,25 @@ def test_block_svd_zero_columns_and_non_finite_blocks_take_the_general_kernel():
     _check(c, *good)
 
 
+@pytest.mark.parametrize("n", [24, 70, 150])
+@pytest.mark.parametrize("decades", [130, 138, 150, 165])
+def test_block_svd_vanishing_columns(n, decades):
+    """Orthogonal columns scaled down to 1e-130 .. 1e-165 of the largest: squared norms that leave
+    the normal range must not cost a factor its orthogonality.  The singular values (the
+    scales) and both factors are right to rounding, or the call says it did not converge
+    (columns below 1e-154, whose squared norms are subnormal)."""
+    rng = np.random.default_rng(n)
+    q = np.linalg.qr(rng.standard_normal((n, n)))[0]
+    d = 10.0 ** (-float(decades) * np.arange(n) / (n - 1))
+    try:
+        ((U, s, Vt),) = _svd_dev([q * d[rng.permutation(n)]])
+    except capi.DmrgError as e:
+        assert e.status == capi.NUMERIC and decades > 150
+        return
+    assert np.max(np.abs(s / d - 1.0)) <= TOL
+    assert np.max(np.abs(U.T @ U - np.eye(n))) <= TOL and np.max(np.abs(Vt @ Vt.T - np.eye(n))) <= TOL
+
+
 def test_block_svd_rejects_null_blocks():
     rows = np.array([2], dtype=np.uint32)
     nul = (capi.C.c_void_p * 1)(None)
