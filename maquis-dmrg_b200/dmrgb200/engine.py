@@ -168,9 +168,11 @@ def schedule_right_step(phys, left, right, mpo: MPOHandle, R: BIndex, symmetric=
 
 # ---- device side --------------------------------------------------------------------
 
-def _view(addresses: np.ndarray):
-    """Boundary view over an array of addresses (0: no storage); the array is returned to be
-    kept alive as long as the view."""
+def _view(addresses):
+    """Boundary view over an array or sequence of addresses (0 or None: no storage); the array
+    is returned to be kept alive as long as the view."""
+    if not isinstance(addresses, np.ndarray) or addresses.dtype.kind not in "iu":
+        addresses = np.array([int(a) if a else 0 for a in addresses], dtype=np.uint64)
     arr = np.ascontiguousarray(addresses, dtype=np.uint64)
     v = capi.BoundaryView()
     v.n_cohorts = len(arr)

@@ -80,6 +80,24 @@ def test_noalloc_rejects_plans_beyond_its_static_area():
     del keep
 
 
+@pytest.mark.parametrize("addresses", [
+    [0x1000, None, 0x3000], (0x1000, 0, 0x3000), np.array([0x1000, 0, 0x3000], np.uint64),
+    np.array([0x1000, 0, 0x3000], np.int64), np.array([0x1000, None, 0x3000], object),
+    np.array([0x1000, 7, 0, 7, 0x3000, 7], np.uint64)[::2], [C.c_uint64(0x1000).value, None, 0x3000]])
+def test_boundary_views_take_arrays_and_lists_with_gaps(addresses):
+    from dmrgb200 import engine as E
+    view, keep = E._view(addresses)
+    assert view.n_cohorts == 3
+    assert [view.cohort_ptr[i] for i in range(3)] == [0x1000, None, 0x3000]
+    del keep
+
+
+def test_boundary_view_of_no_cohorts():
+    from dmrgb200 import engine as E
+    for empty in ([], np.zeros(0, np.uint64)):
+        assert E._view(empty)[0].n_cohorts == 0
+
+
 def test_library_exports_every_declared_entry_point():
     """Every function include/dmrgb200.h declares is exported by libdmrgb200.so and has
     a ctypes signature in the binding (loading needs no GPU)."""
