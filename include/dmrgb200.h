@@ -240,8 +240,11 @@ dmrgb200_status dmrgb200_hpsi_per_block(dmrgb200_plan_t plan, const double* x, d
  * a plan of at least 50 MFLOP per H·psi does this by itself (environment
  * DMRGB200_AUTOTUNE=0 keeps the default variant; plans of small blocks that run as chained
  * products have no GEMM stages to tune); this call re-tunes now, using x (in layout) and y (out
- * layout, overwritten), and returns the chosen variant per stage.  No
- * counterpart in the reference (its cuBLAS calls are untuned). */
+ * layout, overwritten), returns the chosen variant per stage and ends a pin of
+ * dmrgb200_plan_set_gemm_variants.  A plan that runs as chained products does so
+ * afterwards too; the variants then serve its calls that need T or S (the adjoint, an
+ * output that overlaps the input).  No counterpart in the reference (its cuBLAS calls are
+ * untuned). */
 dmrgb200_status dmrgb200_plan_autotune(dmrgb200_plan_t plan, const double* x, double* y, void* cuda_stream,
                                        int32_t variants[2]);
 const char* dmrgb200_gemm_variant_name(int variant);
@@ -250,7 +253,7 @@ int dmrgb200_gemm_variant_count(void);
 /* Pin the grouped-GEMM variant of stage 1 and of stage 3 of an H·psi plan (each 0 ..
  * dmrgb200_gemm_variant_count() - 1) instead of the autotuner's choice: later calls use
  * them and do not tune the plan (dmrgb200_plan_autotune re-tunes); a plan of small blocks,
- * which otherwise runs as chained products in one launch, runs its stages from then on.  The sums are the same
+ * which otherwise runs as chained products in one launch, runs its stages while pinned.  The sums are the same
  * for every variant up to the order of the K steps.  No counterpart in the reference. */
 dmrgb200_status dmrgb200_plan_set_gemm_variants(dmrgb200_plan_t plan, int32_t stage1, int32_t stage3);
 

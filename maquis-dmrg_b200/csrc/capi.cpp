@@ -877,6 +877,7 @@ dmrgb200_status dmrgb200_plan_autotune(dmrgb200_plan_t plan, const double* x, do
                                  plan->S, st);
     drop_variant_graphs(plan);
     if (e != cudaSuccess) return cuda_fail(e, "grouped GEMM autotuning");
+    plan->prog.chained = plan->prog.chain_built;  // a pin ends here
     if (variants) {
         variants[0] = plan->prog.var1;
         variants[1] = plan->prog.var3;

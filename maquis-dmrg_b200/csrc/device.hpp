@@ -204,7 +204,8 @@ struct DeviceProgram {
     // the whole plan as chained products (chained): what the native FP64 H psi and the boundary
     // steps run then; the stages stay for the callers that need T or S (emulated and per-block
     // H psi, adjoint, alpha_dm) and for pinned GEMM variants
-    bool chained = false;
+    bool chained = false;    // what runs: chain_built, unless GEMM variants are pinned
+    bool chain_built = false;
     ChainList chain;
     ChainDev d_chain;
     // stage 3 with long K ranges split over CTAs (own3): what the native FP64 H psi and the

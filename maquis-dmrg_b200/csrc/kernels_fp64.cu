@@ -1373,7 +1373,7 @@ void compile_program(FlatPlan const& p, std::vector<uint64_t> const& stage3_bnd,
     // ---- the whole plan as chained products (the general entry points; not where an S-build form
     // is forced) ----
     if (stack_rows && group_lines && mode == 0 && ug_units.empty())
-        prog.chained = build_chain(p, stage3_bnd, stage1_bnd, outptr, prog.chain);
+        prog.chained = prog.chain_built = build_chain(p, stage3_bnd, stage1_bnd, outptr, prog.chain);
     // ---- stage 3 with long K ranges split ----
     if (stack_rows && group_lines && g3.tiles.size() < 4 * 4 * 148) {
         prog.split_steps = split_target(g3);

@@ -1,6 +1,6 @@
-"""Failed allocations inside the entry points, without a GPU: the library runs in a child
-process whose CUDA runtime calls go to a host stand-in (fake_cudart.c) that records kernel
-launches and fails the allocation it is told to."""
+"""Host logic of the entry points without a GPU, failed allocations among it: the library runs
+in a child process whose CUDA runtime calls go to a host stand-in (fake_cudart.c) that
+records kernel launches and fails the allocation it is told to."""
 import json
 import os
 import subprocess
@@ -133,3 +133,23 @@ print(json.dumps({"want": want, "rows": rows}))
     assert rows[-1][0] == 0 and len(rows) > 8
     for status, later, leaked in rows[:-1]:
         assert status == 3 and later == want and leaked == 0
+
+
+def test_autotuning_ends_a_pin(fake):
+    """Pinned variants replace a plan's chained products by its stages; autotuning the plan
+    brings the one launch back, from device and from host buffers."""
+    got = child(fake, PLAN + """
+p = make()
+a = x.ctypes.data, y.ctypes.data
+dev = lambda: (fake.fake_clear(), p.hpsi(*a), launched())[-1]
+host = lambda: (fake.fake_clear(), p.hpsi_host(*a), launched())[-1]
+out = [dev(), host()]
+p.set_gemm_variants(0, 0)
+out += [dev(), host()]
+capi.check(capi.lib.dmrgb200_plan_autotune(p.handle, *a, None, None), "autotune")
+out += [dev(), host()]
+print(json.dumps(out))
+""")
+    dev, host, pinned, pinned_host, again, again_host = got
+    assert len(dev) == 1 and len(pinned) > 1 and pinned_host != host
+    assert again == dev and again_host == host
