@@ -135,6 +135,14 @@ struct dmrgb200_plan_s {
     double* step_T = nullptr;
     double* step_S = nullptr;
     int* step_err = nullptr;  // pinned: the program's wait-timeout word after a step
+    // T and S of the stages: a step that runs as chained products needs neither
+    cudaError_t step_scratch() {
+        cudaError_t e = cudaSuccess;
+        if (!step_T && step_prog.t_elems) e = cudaMalloc(&step_T, step_prog.t_elems * sizeof(double));
+        if (e == cudaSuccess && !step_S && step_prog.s_elems)
+            e = cudaMalloc(&step_S, step_prog.s_elems * sizeof(double));
+        return e;
+    }
     void drop_step() {
         if (step_valid) free_program(step_prog);
         cudaFree(step_T);
@@ -357,21 +365,16 @@ dmrgb200_status run_step(dmrgb200_plan_s* p, const double* ket, const double* br
             p->step_in_place = p->step_in_place || p->reads.meets(at, n);
         }
         p->step_writes.close();
-        if (p->step_prog.t_elems && (e = cudaMalloc(&p->step_T, p->step_prog.t_elems * sizeof(double))) != cudaSuccess) {
-            p->drop_step();
-            return cuda_fail(e, "step T scratch");
-        }
-        if (p->step_prog.s_elems && (e = cudaMalloc(&p->step_S, p->step_prog.s_elems * sizeof(double))) != cudaSuccess) {
-            p->drop_step();
-            return cuda_fail(e, "step S scratch");
-        }
         static const bool tune = [] {
             const char* v = std::getenv("DMRGB200_AUTOTUNE");
             return !(v && v[0] == '0');
         }();
+        if (!p->step_prog.chained && (e = p->step_scratch()) != cudaSuccess) {
+            p->drop_step();
+            return cuda_fail(e, "step scratch");
+        }
         // (tuning writes the outputs before the step has read its inputs)
-        const bool over = overlaps();
-        if (tune && !p->step_prog.chained && !over && p->flat.flops() >= 50000000ull && !capturing(stream)) {
+        if (tune && !p->step_prog.chained && !overlaps() && p->flat.flops() >= 50000000ull && !capturing(stream)) {
             // the variants run the whole step (outputs included): the run below rewrites them
             if ((e = tune_program(p->step_prog, reinterpret_cast<uint64_t>(ket), reinterpret_cast<uint64_t>(bra),
                                   p->step_T, p->step_S, stream)) != cudaSuccess) {
@@ -380,8 +383,10 @@ dmrgb200_status run_step(dmrgb200_plan_s* p, const double* ket, const double* br
             }
         }
     }
+    const bool staged = !p->step_prog.chained || overlaps();
+    if (staged && (e = p->step_scratch()) != cudaSuccess) return cuda_fail(e, "step scratch");
     e = run_program(p->step_prog, reinterpret_cast<uint64_t>(ket), reinterpret_cast<uint64_t>(bra), p->step_T,
-                    p->step_S, stream, p->timing ? p->ev : nullptr, p->step_prog.chained && overlaps());
+                    p->step_S, stream, p->timing ? p->ev : nullptr, staged);
     // the wait-timeout word comes back with the step's own synchronisation
     const bool word = p->step_prog.d_err != nullptr;
     if (word && !p->step_err && cudaHostAlloc(&p->step_err, sizeof(int), cudaHostAllocDefault) != cudaSuccess)
@@ -1069,17 +1074,8 @@ dmrgb200_status dmrgb200_step_alpha_dm(dmrgb200_plan_t plan, const double* ket, 
         }
         plan->step_valid = true;
         plan->step_outp = placeholder;
-        if (plan->step_prog.t_elems &&
-            (e = cudaMalloc(&plan->step_T, plan->step_prog.t_elems * sizeof(double))) != cudaSuccess) {
-            plan->drop_step();
-            return cuda_fail(e, "alpha_dm T scratch");
-        }
-        if (plan->step_prog.s_elems &&
-            (e = cudaMalloc(&plan->step_S, plan->step_prog.s_elems * sizeof(double))) != cudaSuccess) {
-            plan->drop_step();
-            return cuda_fail(e, "alpha_dm S scratch");
-        }
     }
+    if ((e = plan->step_scratch()) != cudaSuccess) return cuda_fail(e, "alpha_dm scratch");
     if (!plan->dm_valid || plan->dm_ptrs != ptrs) {
         plan->drop_dm();
         GemmList gl;

@@ -232,6 +232,42 @@ struct ChainProblem {
     uint64_t work;
 };
 
+// Where the chain is faster than the three launches, both measured, in us: Hubbard m = 100 6.9
+// against 15.0, 200 7.7 / 17, 333 12.6 / 20.3, 480 20.5 / 28 (blocks of at most 25 rows), 700 45
+// / 42 (36 rows), 1024 85 / 63; Heisenberg m = 64 7.0 / 12.2, 200 16.4 / 18 (30 rows).  Larger
+// blocks keep the pipe busier through shared memory, and computing T anew for every term that
+// reads it starts to cost.  Read off the plan's sizes before anything is built: most plans that
+// are too large are so by these.
+bool chain_sizes(FlatPlan const& p) {
+    const bool left = p.kind == KIND_LEFT;
+    uint64_t tiles = 0;
+    auto problem = [&](uint32_t M, uint32_t N) {
+        tiles += (N + 7) / 8;
+        return M <= CH_TILE;
+    };
+    std::vector<char> written(p.out_rows.size(), 0);
+    for (uint32_t c = 0; c < p.n_cohorts(); ++c) {
+        const bool first = p.kind != KIND_HPSI || !written[p.c_rb[c]];
+        if (p.kind == KIND_HPSI) {
+            written[p.c_rb[c]] = 1;
+        } else {
+            for (uint32_t b = 0; b < p.c_nsrows[c]; ++b)
+                if (!problem(left ? p.c_ls[c] : p.c_rs[c], left ? p.c_rs[c] : p.c_ls[c])) return false;
+        }
+        for (uint32_t u = p.c_unit[c]; u < p.c_unit[c + 1]; ++u) {
+            if (!p.u_ms[u]) continue;
+            if (p.kind == KIND_HPSI && first && !problem(p.out_rows[p.c_rb[c]], p.u_ms[u])) return false;
+            const uint32_t K1 = p.kind == KIND_HPSI ? p.c_ls[c] : p.u_ms[u];
+            if (K1 > CH_TILE)
+                for (uint32_t l = p.u_line[u]; l < p.u_line[u + 1]; ++l)
+                    if (p.l_term[l] < p.l_term[l + 1]) return false;
+        }
+    }
+    for (uint32_t ob = 0; p.kind == KIND_HPSI && ob < p.out_rows.size(); ++ob)
+        if (!written[ob] && !problem(p.out_rows[ob], p.out_cols[ob])) return false;
+    return tiles <= 148 * 16;
+}
+
 }  // namespace
 
 bool build_chain(FlatPlan const& p, std::vector<uint64_t> const& stage3_bnd, std::vector<uint64_t> const& stage1_bnd,
@@ -240,7 +276,7 @@ bool build_chain(FlatPlan const& p, std::vector<uint64_t> const& stage3_bnd, std
     const uint32_t nc = p.n_cohorts();
     const bool left = p.kind == KIND_LEFT;
     // lines of few terms only: the chain computes a term's T anew for every line that reads it
-    if (!nc || p.n_terms() > 4ull * p.n_lines()) return false;
+    if (!nc || p.n_terms() > 4ull * p.n_lines() || !chain_sizes(p)) return false;
     // units of every cohort by offset; they must tile the cohort's S
     std::vector<std::vector<uint32_t>> units(nc);
     for (uint32_t c = 0; c < nc; ++c) {
@@ -388,21 +424,10 @@ bool build_chain(FlatPlan const& p, std::vector<uint64_t> const& stage3_bnd, std
         cl = ChainList();
         return false;
     }
-    // Where the chain is faster than the three launches, both measured, in us: Hubbard m = 100 6.9
-    // against 15.0, 200 7.7 / 17, 333 12.6 / 20.3, 480 20.5 / 28 (blocks of at most 25 rows), 700 45
-    // / 42 (36 rows), 1024 85 / 63; Heisenberg m = 64 7.0 / 12.2, 200 16.4 / 18 (30 rows).  Larger
-    // blocks keep the pipe busier through shared memory, and computing T anew for every term that
-    // reads it starts to cost.
-    uint32_t dmax = 0;
-    uint64_t tiles = 0;
-    for (auto const& pr : probs) {
-        dmax = std::max(dmax, pr.M);
-        tiles += (pr.N + 7) / 8;
-    }
-    for (auto const& L : all_lines) dmax = std::max(dmax, L.k1);
     for (uint32_t t = 0; t < p.n_t(); ++t) staged += p.t_size(t) * (left ? p.t_bcols[t] : p.t_brows[t]);
     for (uint32_t c = 0; c < nc; ++c) staged += uint64_t(p.c_ls[c]) * p.c_nsrows[c] * p.c_rs[c] * p.c_stripe[c];
-    if (probs.empty() || dmax > CH_TILE || tiles > 148 * 16 || macs > 2 * staged) {
+    // T computed anew for every term that reads it must not outweigh the stages' work
+    if (probs.empty() || macs > 2 * staged) {
         cl = ChainList();
         return false;
     }
@@ -467,6 +492,10 @@ bool build_chain(FlatPlan const& p, std::vector<uint64_t> const& stage3_bnd, std
     // 10.4 us whole, 6.9 in four; Hubbard m = 200: 11.4 and 7.7; m = 480: 26.4 whole, 20.5 in
     // two, 26.3 in four).
     cl.blocks = std::max(2, int((std::max(d1, dm) + 7) / 8));
+    if (cl.blocks > int(CH_TILE / 8)) {  // chain_sizes has seen to it
+        cl = ChainList();
+        return false;
+    }
     cl.split = cl.tiles.size() < 148 * 6 ? 4 : cl.tiles.size() < 148 * 10 ? 2 : 1;
     return true;
 }

@@ -768,19 +768,34 @@ std::vector<uint64_t> s_offsets(FlatPlan const& p, uint64_t* total) {
 namespace {
 // Blocks of every T task that some term reads; the others are never used (at the middle
 // of a Fermi-Hubbard chain the tasks hold 2312 blocks of which 1624 are read).
-std::vector<std::vector<char>> t_blocks_read(FlatPlan const& p) {
-    std::vector<std::vector<char>> read(p.n_t());
-    for (uint32_t t = 0; t < p.n_t(); ++t) read[t].assign(p.t_nb[t], 0);
-    for (uint32_t u = 0; u < p.n_units(); ++u)
-        for (uint32_t l = p.u_line[u]; l < p.u_line[u + 1]; ++l)
-            for (uint32_t k = p.l_term[l]; k < p.l_term[l + 1]; ++k) {
-                // columns term_col .. + u_ms of the task's T, usually one whole block
-                const uint32_t t = p.term_t[k], w = p.t_bcols[t];
-                if (!w || !p.u_ms[u]) continue;
-                for (uint32_t b = p.term_col[k] / w; b <= (p.term_col[k] + p.u_ms[u] - 1) / w && b < p.t_nb[t]; ++b)
-                    read[t][b] = 1;
-            }
-    return read;
+struct BlocksRead {
+    std::vector<uint64_t> first;  // per task: its flags in `flag`
+    std::vector<char> flag;
+    const char* of(uint32_t t) const { return flag.data() + first[t]; }
+};
+BlocksRead t_blocks_read(FlatPlan const& p) {
+    BlocksRead r;
+    r.first.resize(p.n_t());
+    uint64_t n = 0;
+    for (uint32_t t = 0; t < p.n_t(); ++t) {
+        r.first[t] = n;
+        n += p.t_nb[t];
+    }
+    r.flag.assign(n, 0);
+    for (uint32_t u = 0; u < p.n_units(); ++u) {
+        const uint32_t ms = p.u_ms[u];
+        if (!ms) continue;
+        const uint32_t k1 = p.u_line[u] < p.u_line[u + 1] ? p.l_term[p.u_line[u + 1]] : 0;
+        for (uint32_t k = k1 ? p.l_term[p.u_line[u]] : 0; k < k1; ++k) {
+            // columns term_col .. + ms of the task's T, usually one whole block
+            const uint32_t t = p.term_t[k], w = p.t_bcols[t], col = p.term_col[k];
+            if (!w) continue;
+            char* f = r.flag.data() + r.first[t];
+            uint32_t b = col / w;
+            for (uint32_t end = b * w; end < col + ms && b < p.t_nb[t]; end += w) f[b++] = 1;
+        }
+    }
+    return r;
 }
 
 // Stage 1 of H psi / right step with the rows of all T tasks that share a
@@ -802,7 +817,7 @@ void stack_stage1(FlatPlan const& p, std::vector<uint64_t> const& stage1_bnd, st
     std::map<std::tuple<uint32_t, uint8_t, uint32_t, uint32_t, uint32_t>, std::vector<uint32_t>> groups;
     for (uint32_t t = 0; t < p.n_t(); ++t)
         if (!keep || (*keep)[t]) groups[{p.t_ci[t], p.t_trans[t], p.t_brows[t], p.t_bcols[t], p.t_nb[t]}].push_back(t);
-    std::vector<std::vector<char>> read;
+    BlocksRead read;
     if (skip_unread) read = t_blocks_read(p);
     auto problem = [&](std::vector<uint32_t> const& tasks, uint32_t b0, uint32_t nb) {
         const uint32_t t0 = tasks.front();
@@ -855,24 +870,34 @@ void stack_stage1(FlatPlan const& p, std::vector<uint64_t> const& stage1_bnd, st
             problem(kv.second, 0, nb);
             continue;
         }
-        std::map<std::vector<char>, std::vector<uint32_t>> by_set;
-        for (uint32_t t : kv.second) by_set[read[t]].push_back(t);
         auto rows = [&](std::vector<uint32_t> const& tasks) {
             uint64_t M = 0;
             for (uint32_t t : tasks) M += p.in_rows[p.t_lb[t]];
             return M;
         };
+        const uint64_t M = rows(kv.second), w32 = steps(t0, 32, M, nb), w64 = steps(t0, 64, M, nb);
+        // the elements read fill so many tiles of 32 x 64 at least
+        uint64_t used = 0;
+        for (uint32_t t : kv.second)
+            used += uint64_t(std::count(read.of(t), read.of(t) + nb, 1)) * p.in_rows[p.t_lb[t]];
+        if (10 * used * p.t_bcols[t0] * ((p.t_brows[t0] + 15) / 16) > 9 * w32 * (32 * 64)) {
+            problem(kv.second, 0, nb);
+            continue;
+        }
+        std::map<std::string, std::vector<uint32_t>> by_set;
+        for (uint32_t t : kv.second) by_set[std::string(read.of(t), nb)].push_back(t);
         std::vector<Piece> pieces;
         uint64_t c32 = 0, c64 = 0;
         for (auto const& sv : by_set) {
-            const uint64_t M = rows(sv.second);
+            const uint64_t Ms = rows(sv.second);
             for (uint32_t b = 0; b < nb;) {
                 uint32_t e = b;
                 while (e < nb && sv.first[e]) ++e;
                 if (e > b) {
                     // over a gap to the run before, where the wider problem has no more tiles
                     if (!pieces.empty() && pieces.back().tasks == &sv.second &&
-                        steps(t0, 32, M, e - pieces.back().b0) <= steps(t0, 32, M, pieces.back().nb) + steps(t0, 32, M, e - b))
+                        steps(t0, 32, Ms, e - pieces.back().b0) <=
+                            steps(t0, 32, Ms, pieces.back().nb) + steps(t0, 32, Ms, e - b))
                         pieces.back().nb = e - pieces.back().b0;
                     else
                         pieces.push_back({&sv.second, b, e - b});
@@ -884,8 +909,7 @@ void stack_stage1(FlatPlan const& p, std::vector<uint64_t> const& stage1_bnd, st
             c32 += steps(t0, 32, rows(*x.tasks), x.nb);
             c64 += steps(t0, 64, rows(*x.tasks), x.nb);
         }
-        const uint64_t M = rows(kv.second);
-        if (10 * c32 > 9 * steps(t0, 32, M, nb) || 10 * c64 > 9 * steps(t0, 64, M, nb)) {
+        if (10 * c32 > 9 * w32 || 10 * c64 > 9 * w64) {
             problem(kv.second, 0, nb);
             continue;
         }

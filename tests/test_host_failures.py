@@ -153,3 +153,74 @@ print(json.dumps(out))
     dev, host, pinned, pinned_host, again, again_host = got
     assert len(dev) == 1 and len(pinned) > 1 and pinned_host != host
     assert again == dev and again_host == host
+
+
+STEP = """
+from helpers import make_chain
+from test_lowering import step_plan
+model, bonds, _, _ = make_chain("hubbard", 12, 0, seed=1, synthetic_m={m})
+plan = step_plan(model, bonds, 4, True)
+assert bool(E.lowering(plan).chained) == {chained}
+store = np.zeros(1 << 20)
+nt, nc = int(plan["t_ci"].max()) + 1, int(plan["c_out_ci"].max()) + 1
+far = np.full(nc, store.ctypes.data + (1 << 22), np.uint64) + 64 * np.arange(nc, dtype=np.uint64)
+ket = np.zeros(int(plan["in_size"]))
+bra = np.zeros(int(plan["out_size"]))
+make = lambda: E.DevicePlan(E.Context(0), plan, left_addr=np.full(nt, store.ctypes.data, np.uint64))
+run = lambda p, out=far: p.step(ket.ctypes.data, bra.ctypes.data, out)
+"""
+
+
+@pytest.mark.parametrize("m,chained", [(60, True), (700, False)])
+def test_step_after_a_failed_allocation(fake, m, chained):
+    """Whichever allocation of a step fails, the next call runs it as a fresh plan does, and
+    destroying the plan gives everything back."""
+    got = child(fake, STEP.format(m=m, chained=chained) + """
+p = make()
+fake.fake_clear()
+run(p)
+want = launched()
+del p
+rows = []
+for k in range(1, 60):
+    before = fake.fake_live()
+    p = make()
+    fake.fake_fail_in(k)
+    status = 0
+    try:
+        run(p)
+    except capi.DmrgError as e:
+        status = e.status
+    fake.fake_fail_in(0)
+    launched()
+    run(p)
+    rows.append([status, launched()])
+    del p
+    rows[-1].append(fake.fake_live() - before)
+    if status == 0:
+        break
+print(json.dumps([want, rows]))
+""")
+    want, rows = got
+    assert (len(want) == 1) == chained
+    assert rows[-1][0] == 0 and len(rows) >= (2 if chained else 4)
+    for status, later, leaked in rows[:-1]:
+        assert status == 3 and later == want and leaked == 0
+
+
+def test_chained_step_over_its_input_runs_the_stages(fake):
+    """A chained step whose output overlaps its ket or its boundary runs the stages, with
+    their scratch allocated then; the next call elsewhere is one launch again."""
+    got = child(fake, STEP.format(m=60, chained=True) + """
+p = make()
+out = []
+for addr in (far, np.full(nc, ket.ctypes.data, np.uint64), far, np.full(nc, store.ctypes.data, np.uint64), far):
+    a = fake.fake_allocations()
+    fake.fake_clear()
+    run(p, addr)
+    out.append([len(launched()), fake.fake_allocations() - a])
+print(json.dumps(out))
+""")
+    (n0, a0), (n1, a1), (n2, _), (n3, a3), (n4, _) = got
+    assert n0 == n2 == n4 == 1 and n1 >= 3 and n3 >= 3
+    assert a1 == a3 == a0 + 2  # T and S

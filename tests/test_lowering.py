@@ -69,3 +69,65 @@ def test_lattice_stage1_leaves_unread_blocks_out(model, width, m, i, share):
     bonds = S.synthetic_bonds(model.phys, len(model.mpo), model.total_charge, m, width)
     form = E.lowering(hpsi_plan(model, bonds, i))
     assert not form.chained and form.stage1_steps <= share * form.stage1_steps_whole
+
+
+def chain_limits(p):
+    """Largest block dimension (rows of the output, K1) and number of eight-column tiles that a
+    plan's chained form has, restated from the plan's arrays."""
+    kind, dmax, tiles = p["kind"], 0, 0
+    left = kind == capi.PLAN_LEFT
+    seen = set()
+    for c in range(len(p["c_lb"])):
+        ls, rs = int(p["c_ls"][c]), int(p["c_rs"][c])
+        rb = int(p["c_rb"][c])
+        for u in range(p["c_unit"][c], p["c_unit"][c + 1]):
+            ms = int(p["u_ms"][u])
+            lines = range(p["u_line"][u], p["u_line"][u + 1])
+            if ms and any(p["l_term"][x] < p["l_term"][x + 1] for x in lines):
+                dmax = max(dmax, ls if kind == capi.PLAN_HPSI else ms)
+            if kind == capi.PLAN_HPSI and rb not in seen and ms:
+                tiles += (ms + 7) // 8
+                dmax = max(dmax, int(p["out_rows"][rb]))
+        seen.add(rb)
+        if kind != capi.PLAN_HPSI:
+            dmax = max(dmax, ls if left else rs)
+            tiles += int(p["c_nsrows"][c]) * (((rs if left else ls) + 7) // 8)
+    if kind == capi.PLAN_HPSI:
+        for ob in set(range(len(p["out_rows"]))) - seen:
+            dmax = max(dmax, int(p["out_rows"][ob]))
+            tiles += (int(p["out_cols"][ob]) + 7) // 8
+    return dmax, tiles
+
+
+def step_plan(model, bonds, i, left):
+    L, phys = len(model.mpo), model.phys
+    handle = lambda p: M.MPOHandle(model.mpo[p], model.symm)
+    idx = E.edge_bindex(model.symm, bonds[0] if left else bonds[L])
+    build = E.schedule_left_step if left else E.schedule_right_step
+    for p in (range(i) if left else range(L - 1, i, -1)):
+        _, idx = build(phys, bonds[p], bonds[p + 1], handle(p), idx, True)
+    return build(phys, bonds[i], bonds[i + 1], handle(i), idx, True)[0].plan
+
+
+@pytest.mark.parametrize("name,L,width", [("heisenberg", 20, 10.0), ("heisenberg", 20, 3.5), ("hubbard", 16, 3.5),
+                                          ("hubbard", 64, 3.5), ("bose", 10, 3.5)])
+def test_plans_run_chained_exactly_within_the_limits(name, L, width):
+    """Blocks of at most 32 rows (K1 too) in at most 2368 tiles, on both sides of each limit, for
+    H·psi and both steps."""
+    from dmrgb200 import mps as S
+    model = {"heisenberg": M.heisenberg, "hubbard": M.fermi_hubbard, "bose": lambda n: M.bose_hubbard(n, N=n // 2)}[name](L)
+    got = set()
+    sizes = sorted({int(round(8 * 1.3 ** k)) for k in range(22)} | {40 * k for k in range(1, 30)}) if L < 64 else (400, 560, 600, 900)
+    for m in sizes:
+        bonds = S.synthetic_bonds(model.phys, L, model.total_charge, m, width)
+        i = L // 2 - 1
+        for p in (hpsi_plan(model, bonds, i), step_plan(model, bonds, i, True), step_plan(model, bonds, i, False)):
+            form = E.lowering(p)
+            dmax, tiles = chain_limits(p)
+            if not tiles:
+                continue
+            few = len(p["term_alpha"]) <= 4 * len(p["l_b1"])
+            assert bool(form.chained) == (few and dmax <= 32 and tiles <= 2368), (m, p["kind"], dmax, tiles)
+            assert not form.chained or form.chain_tiles == tiles
+            got.add(bool(form.chained))
+    assert got == {True, False} or name == "bose"
