@@ -100,7 +100,11 @@ __device__ __forceinline__ int swz(int k) { return (k >> 2) & 3; }
 // stored.  A whole K step has no per-copy conditions (about five instructions per copy
 // instead of ten: on blocks of 17 to 52 rows the copies' arithmetic is most of what the
 // kernel executes); the last one of a segment zero-fills its K rows past the end, in the half
-// or the whole stage that is multiplied.
+// or the whole stage that is multiplied.  Eight-deep stages have so few copies each that the
+// two forms and the running address (each copy's waits for the one before) cost more than the
+// conditions: there every copy has its own, in one loop for both layouts
+// (tile16x64_k8_stages3_ctas6 on stage 3 of Heisenberg m = 230, 300, 400: H psi 19.8, 22.5, 28.0
+// us in the two forms, 17.4, 19.5, 23.8 this way).
 struct CopyStream {
     const char* base;
     const char* safe;  // a readable address for copies that fetch nothing
@@ -113,7 +117,16 @@ struct CopyStream {
 template <int ROWS, int BK_, int NTHREADS, int LD>
 __device__ __forceinline__ void issue_copies(double* tile, CopyStream& cs, uint32_t krem) {
     constexpr int NC = ROWS * BK_ / NTHREADS;
-    if (cs.rowmajor) {
+    if (BK_ < 16) {
+        constexpr int KJ = NTHREADS / ROWS, RJ = NTHREADS / BK_;
+#pragma unroll
+        for (int j = 0; j < NC; ++j) {
+            const uint32_t k = cs.rowmajor ? cs.kt + j * KJ : cs.kt, r = cs.rowmajor ? cs.r : cs.r + j * RJ;
+            const bool ok = ((cs.mask >> j) & 1u) && k < krem;
+            cp_async8(&tile[k * LD + (r ^ swz(k))], reinterpret_cast<const double*>(ok ? cs.base + j * cs.jstride : cs.safe),
+                      ok);
+        }
+    } else if (cs.rowmajor) {
         constexpr int KJ = NTHREADS / ROWS;
         static_assert(KJ <= 4 || NC == 1 || KJ % 4 == 0, "swizzle of copy j");
         if (cs.mask) {
@@ -215,7 +228,9 @@ __global__ void __launch_bounds__(NTHREADS, MINB) gemm_f64_grouped(const DevProb
     wait_for_predecessor();
 
     const int tid = threadIdx.x;
-    const int lane = tid & 31, warp = tid >> 5;
+    // one value per warp also to the compiler: branches on the warp's place need no reconvergence
+    // (Heisenberg m = 230 to 400 19.2 to 26.8 us without, 18.8 to 26.4 with)
+    const int lane = tid & 31, warp = __shfl_sync(0xffffffffu, tid >> 5, 0);
     const int wm = (warp % WARPS_M) * WM, wn = (warp / WARPS_M) * WN;
     const int g = lane >> 2, q = lane & 3;
 
