@@ -77,6 +77,12 @@ __global__ void __launch_bounds__(32 * CH_WARPS, MINB)
     asm volatile("griddepcontrol.wait;" ::: "memory");
 
     const int M = int(t.rows), N = int(t.cols), mb = (M + 7) / 8, n_terms = int(t1 - t0);
+    // z: the product of the current term.  The terms of a line before it lie added up in shared
+    // memory (`open`: there are any): each is summed by itself and then added, as T and S are in the
+    // stages.  Adding a small term's products one by one to a large sum would round at the size of
+    // the large one every time (errors against long double up to 1.3 times the stages' on boundary
+    // steps, 0.75 to 0.95 times this way).
+    bool open = false;
     double acc[B][2], z[B][2];
 #pragma unroll
     for (int j = 0; j < B; ++j) acc[j][0] = acc[j][1] = z[j][0] = z[j][1] = 0.0;
@@ -86,7 +92,7 @@ __global__ void __launch_bounds__(32 * CH_WARPS, MINB)
     // inside (their products are not used); K2 rows past the end read zero.
     int kt = 0, s = 0, k2 = 0, kb = 0;
     const double *qp = nullptr, *pp = nullptr;
-    uint64_t qs = 0, ps = 0;
+    uint32_t qs = 0, ps = 0;
     uint32_t ro[B];
     double alpha = 0.0;
     auto enter = [&]() {
@@ -98,18 +104,18 @@ __global__ void __launch_bounds__(32 * CH_WARPS, MINB)
         alpha = T.alpha;
         qp = operand(bases, T.q) + (uint64_t(q) * T.q2 + uint64_t(int(t.n0) + min(g, N - 1)) * T.qn);
         pp = operand(bases, T.p) + uint64_t(q) * T.p2;
-        qs = 4ull * T.q2;
-        ps = 4ull * T.p2;
+        qs = 4u * T.q2;
+        ps = 4u * T.p2;
 #pragma unroll
         for (int x = 0; x < B; ++x) ro[x] = uint32_t(min(8 * x + g, k1 - 1)) * T.p1;
     };
     struct Step {
         double f, p[B];
-        int kb, apply;  // blocks of K1; term whose line ends with this step, or -1
+        int code;  // blocks of K1, and above bit 3 one more than the term that ends with this step (0: none)
     };
     auto load = [&](Step& st) -> bool {
         if (kt >= n_terms) return false;
-        st.kb = kb;
+        st.code = kb;
         if (s + 4 <= k2) {
             st.f = alpha * *qp;
 #pragma unroll
@@ -125,10 +131,8 @@ __global__ void __launch_bounds__(32 * CH_WARPS, MINB)
         s += 4;
         qp += qs;
         pp += ps;
-        st.apply = -1;
         if (s >= k2) {
-            if (rec[kt].last) st.apply = kt;
-            ++kt;
+            st.code |= ++kt << 3;
             s = 0;
             enter();
         }
@@ -137,12 +141,30 @@ __global__ void __launch_bounds__(32 * CH_WARPS, MINB)
     auto consume = [&](Step const& st) {
 #pragma unroll
         for (int x = 0; x < B; ++x) {
-            if (x >= st.kb) break;
+            if (x >= (st.code & 7)) break;
             dmma(z[x], st.f, st.p[x]);
         }
-        if (st.apply < 0) return;
+        if (st.code < 8) return;
+        const DevChainTerm& T = rec[(st.code >> 3) - 1];
+        double(*before)[2][32] = part[warp];
+        if (open) {
+#pragma unroll
+            for (int x = 0; x < B; ++x) {
+                z[x][0] += before[x][0][lane];
+                z[x][1] += before[x][1][lane];
+            }
+        }
+        open = !T.last;
+        if (open) {
+#pragma unroll
+            for (int x = 0; x < B; ++x) {
+                before[x][0][lane] = z[x][0];
+                before[x][1][lane] = z[x][1];
+                z[x][0] = z[x][1] = 0.0;
+            }
+            return;
+        }
         // acc (M x 8) += A z^T, the even and the odd k of every block of eight
-        const DevChainTerm& T = rec[st.apply];
         const int k1 = int(T.k1);
         const double* A = operand(bases, T.a);
         uint32_t ao[B];
@@ -202,13 +224,18 @@ __global__ void __launch_bounds__(32 * CH_WARPS, MINB)
             }
     }
     if (!live) return;
-    double* C = const_cast<double*>(operand(bases, t.c)) + uint64_t(t.n0) * t.cn;
+    // the tile's output is read again here instead of being held in registers through the products
+    uint32_t to = ti;
+    asm volatile("" : "+r"(to));
+    const DevChainTile& o = tiles[to];
+    const uint32_t cm = o.cm, cn = o.cn;
+    double* C = const_cast<double*>(operand(bases, o.c)) + uint64_t(o.n0) * cn;
 #pragma unroll
     for (int j = 0; j < B; ++j)
 #pragma unroll
         for (int e = 0; e < 2; ++e) {
             const int r = 8 * j + g, c = 2 * q + e;
-            if (r < M && c < N) C[uint64_t(r) * t.cm + uint64_t(c) * t.cn] = acc[j][e];
+            if (r < M && c < N) C[uint64_t(r) * cm + uint64_t(c) * cn] = acc[j][e];
         }
 }
 
@@ -233,8 +260,8 @@ struct ChainProblem {
 };
 
 // Where the chain is faster than the three launches, both measured, in us: Hubbard m = 100 6.9
-// against 15.0, 200 7.7 / 17, 333 12.6 / 20.3, 480 20.5 / 28 (blocks of at most 25 rows), 700 45
-// / 42 (36 rows), 1024 85 / 63; Heisenberg m = 64 7.0 / 12.2, 200 16.4 / 18 (30 rows).  Larger
+// against 15.0, 200 7.7 / 17, 333 12.4 / 20.3, 480 19.5 / 28 (blocks of at most 25 rows), 700 45
+// / 42 (36 rows), 1024 85 / 63; Heisenberg m = 64 6.7 / 12.2, 200 16.0 / 18 (30 rows).  Larger
 // blocks keep the pipe busier through shared memory, and computing T anew for every term that
 // reads it starts to cost.  Read off the plan's sizes before anything is built: most plans that
 // are too large are so by these.

@@ -238,3 +238,47 @@ def test_chained_steps_in_place(name, L, m):
                 assert _rel(got[ref != 0.0], ref[ref != 0.0]) <= TOL, (left, p, over)
             idx, val = nidx, ref
     assert chained >= L // 2
+
+
+@pytest.mark.parametrize("large_first", [True, False])
+@pytest.mark.parametrize("staged", [False, True])
+def test_terms_of_a_line_are_summed_one_by_one(large_first, staged):
+    """A line of two terms, one of them 2^30 times a small integer without rounding, the other a
+    sum of 32 products of unit normals: each term is summed by itself, so the only rounding
+    at the size of the large one is that of the sum (half a unit in the last place, 2^-23 below
+    2^31; the small term's own roundings are below 2^-43).  Adding the 32 products one by one to the
+    large term would round 32 times."""
+    u = lambda *v: np.array(v, dtype=np.uint32)
+    ls, k2, n = 8, 32, 8
+    big, small = (0, 1) if large_first else (1, 0)  # column slice and boundary cohort
+    plan = {
+        "kind": 0, "in_size": ls * 2 * k2, "out_size": ls * n, "g_t": u(0, 2), "g_c": u(0, 1),
+        "in_rows": u(ls), "in_cols": u(2 * k2), "in_off": np.array([0], np.uint64),
+        "out_rows": u(ls), "out_cols": u(n), "out_off": np.array([0], np.uint64),
+        "t_lb": u(0, 0), "t_col": u(0, k2), "t_ci": u(0, 1), "t_trans": np.zeros(2, np.uint8), "t_nb": u(1, 1),
+        "t_brows": u(k2, k2), "t_bcols": u(n, n), "t_width": u(),
+        "c_lb": u(0), "c_rb": u(0), "c_ls": u(ls), "c_rs": u(ls), "c_ci": u(0), "c_trans": np.zeros(1, np.uint8),
+        "c_nsrows": u(1), "c_stripe": u(n), "c_out_ci": u(0), "c_unit": u(0, 1),
+        "u_offset": u(0), "u_ms": u(n), "u_line": u(0, 1), "l_b1": u(0), "l_term": u(0, 2),
+        "term_alpha": np.ones(2), "term_t": u(0, 1), "term_col": u(0, 0)}
+    assert E.lowering(plan).chained
+    rng = np.random.default_rng(5)
+    x = np.zeros((2, ls, k2))  # the two slices
+    B = np.zeros((2, k2, n))
+    x[big, :, 0] = rng.integers(1, 2, ls) * 2.0 ** 30
+    B[big, 0, :] = 1.0
+    x[small], B[small] = rng.standard_normal((ls, k2)), rng.standard_normal((k2, n))
+    ctx = E.Context(0)
+    Lb = E.to_device(np.eye(ls).reshape(-1))
+    Rb = E.to_device(B.transpose(0, 2, 1).reshape(-1))  # each block column-major
+    p = E.DevicePlan(ctx, plan, left_addr=np.array([Lb.data_ptr()], np.uint64),
+                     other_addr=np.array([Rb.data_ptr(), Rb.data_ptr() + 8 * k2 * n], np.uint64))
+    if staged:
+        p.set_gemm_variants(0, 0)
+    xd = E.to_device(np.concatenate([x[0].T.reshape(-1), x[1].T.reshape(-1)]))
+    yd = torch.zeros(ls * n, dtype=torch.float64, device="cuda")
+    p.hpsi(xd.data_ptr(), yd.data_ptr())
+    torch.cuda.synchronize()
+    ref = sum(x[i].astype(np.longdouble) @ B[i].astype(np.longdouble) for i in (0, 1))
+    err = np.abs(yd.cpu().numpy().reshape(n, ls).T - ref)
+    assert float(err.max()) <= 2.0 ** -23 * (1 + 2.0 ** -15)
