@@ -134,7 +134,6 @@ struct dmrgb200_plan_s {
     DeviceProgram step_prog;
     double* step_T = nullptr;
     double* step_S = nullptr;
-    int* step_err = nullptr;  // pinned: the program's wait-timeout word after a step
     // T and S of the stages: a step that runs as chained products needs neither
     cudaError_t step_scratch() {
         cudaError_t e = cudaSuccess;
@@ -387,18 +386,19 @@ dmrgb200_status run_step(dmrgb200_plan_s* p, const double* ket, const double* br
     if (staged && (e = p->step_scratch()) != cudaSuccess) return cuda_fail(e, "step scratch");
     e = run_program(p->step_prog, reinterpret_cast<uint64_t>(ket), reinterpret_cast<uint64_t>(bra), p->step_T,
                     p->step_S, stream, p->timing ? p->ev : nullptr, staged);
-    // the wait-timeout word comes back with the step's own synchronisation
+    // the wait-timeout word comes back before the step's own synchronisation.  Into pageable
+    // memory: a pinned word costs a plan 1.5 to 3 ms to allocate, as much as a small step's whole
+    // first call, and most plans of a sweep run one step.
     const bool word = p->step_prog.d_err != nullptr;
-    if (word && !p->step_err && cudaHostAlloc(&p->step_err, sizeof(int), cudaHostAllocDefault) != cudaSuccess)
-        return cuda_fail(cudaErrorMemoryAllocation, "step error word");
+    int err = 0;
     if (word && e == cudaSuccess)
-        e = cudaMemcpyAsync(p->step_err, p->step_prog.d_err, sizeof(int), cudaMemcpyDeviceToHost, stream);
+        e = cudaMemcpyAsync(&err, p->step_prog.d_err, sizeof(int), cudaMemcpyDeviceToHost, stream);
     cudaError_t e2 = cudaStreamSynchronize(stream);
     if (p->timing && e == cudaSuccess && e2 == cudaSuccess) {
         p->pending = true;  // the device time of the three stages, without the host-side lowering
         p->collect();
     }
-    const bool timed_out = word && e == cudaSuccess && e2 == cudaSuccess && *p->step_err && sbuild_timed_out(p->step_prog);
+    const bool timed_out = word && e == cudaSuccess && e2 == cudaSuccess && err && sbuild_timed_out(p->step_prog);
     if (e != cudaSuccess) return cuda_fail(e, "step launch");
     if (e2 != cudaSuccess) return cuda_fail(e2, "step execution");
     if (timed_out) return fail(DMRGB200_TIMEOUT, "step S build: a bulk-copy wait timed out");
@@ -717,7 +717,6 @@ dmrgb200_status dmrgb200_plan_destroy(dmrgb200_plan_t plan) {
     jd_graph_free(plan->jd);
     blas_handle_free(plan->blas);
     plan->drop_step();
-    cudaFreeHost(plan->step_err);
     plan->drop_dm();
     oz_free(plan->oz1);
     oz_free(plan->oz3);
