@@ -325,6 +325,8 @@ bool build_chain(FlatPlan const& p, std::vector<uint64_t> const& stage3_bnd, std
     std::vector<ChainProblem> probs;
     std::vector<Line> all_lines;
     std::vector<Term> all_terms;
+    all_lines.reserve(2 * size_t(p.n_lines()));  // a line is read by one or two problems
+    all_terms.reserve(2 * size_t(p.n_terms()));
     uint64_t macs = 0, staged = 0;
     bool whole = true;  // every term reads one whole T block
     auto add_line = [&](ChainProblem& pr, int64_t l, uint64_t a, uint32_t am, uint32_t ak, uint32_t K1) {
@@ -462,10 +464,17 @@ bool build_chain(FlatPlan const& p, std::vector<uint64_t> const& stage3_bnd, std
     // of all rows and eight columns, the longest problems first
     std::stable_sort(probs.begin(), probs.end(), [](ChainProblem const& a, ChainProblem const& b) { return a.work > b.work; });
     uint32_t d1 = 1, dm = 1;
+    std::vector<uint64_t> cost;  // work up to each line end of a problem
+    std::vector<uint32_t> ends;  // record index there
+    cl.terms.reserve(all_terms.size());
+    uint64_t n_tiles = 0;
+    for (auto const& pr : probs) n_tiles += (pr.N + 7) / 8;
+    cl.tiles.reserve(n_tiles);
+    cl.block_off.reserve(n_tiles);
     for (auto const& pr : probs) {
         const uint32_t begin = uint32_t(cl.terms.size());
-        std::vector<uint64_t> cost{0};       // work up to each line end
-        std::vector<uint32_t> ends{begin};   // record index there
+        cost.assign(1, 0);
+        ends.assign(1, begin);
         for (uint32_t l = pr.line_begin; l < pr.line_end; ++l) {
             Line const& L = all_lines[l];
             d1 = std::max(d1, L.k1);

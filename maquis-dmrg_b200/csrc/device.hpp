@@ -248,7 +248,6 @@ struct DeviceProgram {
     uint32_t n_gitems8 = 0;  // gitems[0, n_gitems8): groups of up to 8 lines (the narrow launch)
     TileLists x1, x3;  // tile lists of the other classes
     DevRow* d_r1 = nullptr;  // stage-1 row table (stacked T tasks)
-    GemmList stage1_tasks;   // stage 1 as one problem per T task (when stage1 is stacked)
     // grouped-GEMM variant per stage (autotuned by tune_program)
     int var1 = 0, var3 = 0;
     bool tuned = false;
@@ -258,8 +257,7 @@ struct DeviceProgram {
 // boundary read by stage 3 (H psi: L) and by stage 1 (H psi, right step: R;
 // left step: L).  outptr: device address of each output boundary cohort (steps).
 // stack_rows: stage 1 of H psi / right step as one row-table problem per set of
-// T tasks that share their boundary cohort (rows of all those tasks stacked);
-// the per-task list is kept in prog.stage1_tasks.
+// T tasks that share their boundary cohort (rows of all those tasks stacked).
 // group_lines: a unit whose lines share enough sources runs its S build as line
 // groups (DevSGroup) when that issues at most twice the multiply-adds of the
 // per-line walk; DMRGB200_SBUILD=lines / groups in the environment forces one

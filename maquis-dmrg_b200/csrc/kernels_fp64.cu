@@ -1213,9 +1213,11 @@ void compile_program(FlatPlan const& p, std::vector<uint64_t> const& stage3_bnd,
     // element past a source row
     prog.t_elems += 32;
 
-    // ---- stage 1 ----
+    // ---- stage 1: rows stacked by boundary cohort, or one problem per T task ----
     GemmList& g1 = prog.stage1;
-    for (uint32_t t = 0; t < nt; ++t) {
+    const bool stacked = stack_rows && p.kind != KIND_LEFT && nt;
+    if (stacked) stack_stage1(p, stage1_bnd, t_off, g1, nullptr, group_lines);
+    for (uint32_t t = 0; !stacked && t < nt; ++t) {
         DevProb pr;
         DevSeg sg{};
         uint64_t bnd = stage1_bnd.at(p.t_ci[t]) / 8;
@@ -1252,11 +1254,7 @@ void compile_program(FlatPlan const& p, std::vector<uint64_t> const& stage3_bnd,
         g1.probs.push_back(pr);
         add_tiles(g1, uint32_t(g1.probs.size() - 1), p.t_nb[t]);
     }
-    sort_tiles(g1);
-    if (stack_rows && p.kind != KIND_LEFT && p.n_t()) {
-        prog.stage1_tasks = std::move(prog.stage1);
-        stack_stage1(p, stage1_bnd, t_off, prog.stage1, nullptr, group_lines);
-    }
+    if (!stacked) sort_tiles(g1);
 
     // ---- stage 2 (S lines) ----
     std::vector<uint64_t> s_off = s_offsets(p, &prog.s_elems);
