@@ -366,6 +366,14 @@ def split_workload(args):
     print(json.dumps(line), flush=True)
 
 
+def check_energies(solves):
+    """The graph-captured and the stepwise solver run the same H·psi and the same iterations: their
+    energies differ by rounding only, or one of them computed something else."""
+    a, b = solves["graph"]["energy"], solves["stepwise"]["energy"]
+    if not abs(a - b) <= 1e-11 * abs(a):
+        raise SystemExit(f"bench: the solvers' energies differ: graph {a!r}, stepwise {b!r}")
+
+
 def solve_workload(args):
     """Jacobi-Davidson solves of the Hubbard L=64 m=1024 site problem (8 iterations each, tol 0 so
     that every iteration runs), graph-captured and stepwise; one JSON line."""
@@ -390,7 +398,8 @@ def solve_workload(args):
                 wall.append((time.perf_counter() - t0) * 1e3)
                 dev.append(st.solve_ms)
         out[name] = {"solve_ms_device": statistics.mean(dev), "solve_ms_wall": statistics.mean(wall),
-                     "iterations": int(st.iterations)}
+                     "iterations": int(st.iterations), "energy": e}
+    check_energies(out)
     hp = sp.plan.flops * 8 / 1e9
     print(json.dumps({"metric": "Jacobi-Davidson solve time (ms, 8 H·psi)", "value": out["graph"]["solve_ms_wall"],
                       "unit": "ms", "higher_is_better": False, "n_gpus": 1, "dtype": "f64", "data": "synthetic",
@@ -1026,6 +1035,7 @@ def main():
         jd[name] = {"solve_ms_device": statistics.mean(t[0] for t in times),
                     "solve_ms_wall": statistics.mean(t[1] for t in times), "iterations": int(st.iterations),
                     "energy": e}
+    check_energies(jd)
     sp.plan.set_solver(capi.SOLVER_GRAPH)
     # the same solve with every H·psi emulated on the INT8 tensor cores: slices tuned so that
     # H·psi of the start vector is within 1e-10 of FP64, energy compared with the FP64 solve

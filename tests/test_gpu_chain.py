@@ -5,6 +5,7 @@ takes up to 32; K1 and rows in blocks of 8, columns in tiles of 8, K2 in steps o
 import numpy as np
 import pytest
 
+from dmrgb200 import _capi as capi
 from dmrgb200 import engine as E
 from dmrgb200 import models as M
 from dmrgb200 import mps as S
@@ -28,17 +29,61 @@ def _plan(ctx, ch):
     return plan, (Lb, Rb)
 
 
+def one_cohort_plan(ls, rs, ns, n, trans):
+    """One T task (x times one block), one cohort of ns MPO rows, every row a multiple of T: y =
+    sum over b of L_b (alpha_b T) with K = ns ls."""
+    u = lambda *v: np.array(v, dtype=np.uint32)
+    rows = np.arange(ns, dtype=np.uint32)
+    return {
+        "kind": 0, "in_size": ls * n, "out_size": rs * n, "g_t": u(0, 1), "g_c": u(0, 1),
+        "in_rows": u(ls), "in_cols": u(n), "in_off": np.array([0], np.uint64),
+        "out_rows": u(rs), "out_cols": u(n), "out_off": np.array([0], np.uint64),
+        "t_lb": u(0), "t_col": u(0), "t_ci": u(0), "t_trans": np.zeros(1, np.uint8), "t_nb": u(1),
+        "t_brows": u(n), "t_bcols": u(n), "t_width": u(),
+        "c_lb": u(0), "c_rb": u(0), "c_ls": u(ls), "c_rs": u(rs), "c_ci": u(0), "c_trans": np.array([trans], np.uint8),
+        "c_nsrows": u(ns), "c_stripe": u(n), "c_out_ci": u(0), "c_unit": u(0, 1),
+        "u_offset": u(0), "u_ms": u(n), "u_line": u(0, ns), "l_b1": rows, "l_term": np.arange(ns + 1, dtype=np.uint32),
+        "term_alpha": np.random.default_rng(7).standard_normal(ns), "term_t": 0 * rows, "term_col": 0 * rows}
+
+
+@pytest.mark.parametrize("trans", [0, 1])
+@pytest.mark.parametrize("ls,rs,ns,n,parts", [(63, 40, 200, 33, 16), (64, 33, 12, 64, 1), (63, 70, 13, 40, 2), (33, 34, 250, 17, 11)])
+def test_split_up_to_the_most_parts(ls, rs, ns, n, parts, trans):
+    """K of 768 (whole) to 12600 (the most parts, 16) in one segment or, transposed, in ns."""
+    plan = one_cohort_plan(ls, rs, ns, n, trans)
+    form = E.lowering(plan)
+    assert not form.chained and (form.stage3_parts == parts or trans)
+    rng = np.random.default_rng(ns)
+    x, B = rng.standard_normal((ls, n)), rng.standard_normal((n, n))
+    L = rng.standard_normal((ns, rs, ls))
+    Lb = E.to_device((L.transpose(0, 1, 2) if trans else L.transpose(0, 2, 1)).reshape(-1))  # column-major blocks
+    Rb, xd = E.to_device(B.T.reshape(-1)), E.to_device(x.T.reshape(-1))
+    p = E.DevicePlan(E.Context(0), plan, left_addr=np.array([Lb.data_ptr()], np.uint64),
+                     other_addr=np.array([Rb.data_ptr()], np.uint64))
+    ref = np.einsum("b,bij->ij", plan["term_alpha"], L.astype(np.longdouble)) @ (x.astype(np.longdouble) @ B)
+    for v in range(capi.lib.dmrgb200_gemm_variant_count()):
+        p.set_gemm_variants(0, v)
+        yd = torch.full((rs * n,), float("nan"), dtype=torch.float64, device="cuda")
+        p.hpsi(xd.data_ptr(), yd.data_ptr())
+        torch.cuda.synchronize()
+        y = yd.cpu().numpy().reshape(n, rs).T
+        # 12600 products whose sum is about a hundredth of the sum of their sizes
+        assert float(np.linalg.norm(y - ref) / np.linalg.norm(ref)) <= 1e-13, v
+
+
 def _rel(a, b):
     return np.linalg.norm(a - b) / np.linalg.norm(b)
 
 
-@pytest.mark.parametrize("name,L,m,i", [("heisenberg", 12, 5, 5), ("heisenberg", 16, 64, 3), ("heisenberg", 20, 80, 9), ("heisenberg", 20, 230, 9),
-                                        ("hubbard", 8, 12, 0), ("hubbard", 12, 60, 5), ("hubbard", 14, 333, 4),
-                                        ("hubbard", 14, 600, 6), ("hubbard", 14, 660, 6), ("bose", 10, 40, 8)])
-def test_chain_matches_oracle_and_stages(name, L, m, i):
+@pytest.mark.parametrize("name,L,m,i,chained", [
+    ("heisenberg", 12, 5, 5, True), ("heisenberg", 16, 64, 3, True), ("heisenberg", 20, 80, 9, True),
+    ("heisenberg", 20, 230, 9, False), ("hubbard", 8, 12, 0, False), ("hubbard", 12, 60, 5, True),
+    ("hubbard", 14, 333, 4, True), ("hubbard", 14, 600, 6, True), ("hubbard", 14, 660, 6, False), ("bose", 10, 40, 8, True)])
+def test_chain_matches_oracle_and_stages(name, L, m, i, chained):
     ctx = E.Context(0)
     model, bonds, tensors, rng = make_chain(name, L, 0, seed=m, synthetic_m=m)
     ch = OracleChain(model, bonds, tensors, i)
+    assert bool(E.lowering(ch.sched.plan).chained) == chained
     plan, keep = _plan(ctx, ch)
     x = random_psi(ch.p12, ch.left, ch.right, rng).data
     xd = E.to_device(x)
@@ -117,8 +162,8 @@ def test_chain_non_finite_boundary_stays_local():
     assert _rel(y[fine], ref[fine]) <= TOL
 
 
-@pytest.mark.parametrize("L,m", [(8, 100), (10, 150)])
-def test_split_stage3_matches_oracle(L, m):
+@pytest.mark.parametrize("L,m,parts", [(8, 100, 1), (10, 150, 3), (12, 200, 6)])
+def test_split_stage3_matches_oracle(L, m, parts):
     """Quantum chemistry in SU2U1 form: few output blocks with long K ranges, cut into parts
     (K of up to a few thousand against parts of at least 48 steps of 16)."""
     ctx = E.Context(0)
@@ -127,6 +172,7 @@ def test_split_stage3_matches_oracle(L, m):
     rng = np.random.default_rng(4)
     tensors = S.random_mps(SU.PHYS, bonds, rng)
     ch = OracleChain(model, bonds, tensors, L // 2 - 1)
+    assert E.lowering(ch.sched.plan).stage3_parts == parts
     plan, keep = _plan(ctx, ch)
     x = rng.standard_normal(int(ch.sched.plan["in_size"]))
     xd = E.to_device(x)
