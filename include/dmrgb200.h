@@ -253,8 +253,9 @@ int dmrgb200_gemm_variant_count(void);
 /* Pin the grouped-GEMM variant of stage 1 and of stage 3 of an H·psi plan (each 0 ..
  * dmrgb200_gemm_variant_count() - 1) instead of the autotuner's choice: later calls use
  * them and do not tune the plan (dmrgb200_plan_autotune re-tunes); a plan of small blocks,
- * which otherwise runs as chained products in one launch, runs its stages while pinned.  The sums are the same
- * for every variant up to the order of the K steps.  No counterpart in the reference. */
+ * which otherwise runs as chained products in one launch, runs its stages while pinned.
+ * The sums are the same for every variant up to the order of the K steps.  No counterpart
+ * in the reference. */
 dmrgb200_status dmrgb200_plan_set_gemm_variants(dmrgb200_plan_t plan, int32_t stage1, int32_t stage3);
 
 /* H·psi with host buffers, the counterpart of the reference's super_hamil_mv on
@@ -262,7 +263,8 @@ dmrgb200_status dmrgb200_plan_set_gemm_variants(dmrgb200_plan_t plan, int32_t st
  * layout, in_size doubles) is copied to the device, y_host (out layout, out_size
  * doubles) receives H·psi.  Stage 1 runs in four parts by input range and stage 3
  * in four parts by output range, so the copies of one range overlap the products
- * of another; the result is bitwise that of dmrgb200_hpsi.  Pin the host buffers
+ * of another (a plan that runs as chained products, one launch that needs all of x,
+ * runs it between two whole copies); the result is bitwise that of dmrgb200_hpsi.  Pin the host buffers
  * (cudaHostAlloc / cudaHostRegister) for the copies to overlap.  Stream-ordered on
  * cuda_stream: synchronise it before reading y_host.  The first call builds the
  * split program and device copies of x and y (kept by the plan); the sequence is

@@ -26,8 +26,7 @@
 // of a K step are in flight while the step before multiplies, across terms; the term records
 // go to shared memory before the wait for the previous kernel.  Where the tiles are too few
 // to fill the SMs, a tile's lines are split over 2 or 4 warps, added in order at the end.
-// Every output element is summed in an order fixed by the plan: bitwise reproducible, and the
-// same in whatever list its tile stands.
+// Every output element is summed in an order fixed by the plan: bitwise reproducible.
 #include <algorithm>
 
 #include "device.hpp"
@@ -253,7 +252,7 @@ struct Line {
 };
 // a problem before it is cut into tiles
 struct ChainProblem {
-    uint64_t c, off;  // output reference; offset of the H psi output block (for ranges)
+    uint64_t c;  // output reference
     uint32_t M, N, cm, cn;
     uint32_t line_begin, line_end;
     uint64_t work;
@@ -399,7 +398,7 @@ bool build_chain(FlatPlan const& p, std::vector<uint64_t> const& stage3_bnd, std
             auto const& cs = by_out[ob];
             const uint32_t M = p.out_rows[ob];
             if (cs.empty()) {  // no cohort writes the block: zeros
-                probs.push_back({ref(BUF_OUT, p.out_off[ob]), p.out_off[ob], M, p.out_cols[ob], 1, M, uint32_t(all_lines.size()),
+                probs.push_back({ref(BUF_OUT, p.out_off[ob]), M, p.out_cols[ob], 1, M, uint32_t(all_lines.size()),
                                  uint32_t(all_lines.size()), 0});
                 continue;
             }
@@ -410,7 +409,7 @@ bool build_chain(FlatPlan const& p, std::vector<uint64_t> const& stage3_bnd, std
                     if (p.u_offset[units[c][x]] != p.u_offset[first[x]]) return false;
             }
             for (size_t x = 0; x < first.size(); ++x) {
-                ChainProblem pr{ref(BUF_OUT, p.out_off[ob] + uint64_t(p.u_offset[first[x]]) * M), p.out_off[ob], M,
+                ChainProblem pr{ref(BUF_OUT, p.out_off[ob] + uint64_t(p.u_offset[first[x]]) * M), M,
                                 p.u_ms[first[x]], 1, M, uint32_t(all_lines.size()), 0, 0};
                 for (uint32_t c : cs) {
                     const uint32_t ls = p.c_ls[c], rs = p.c_rs[c];
@@ -434,7 +433,7 @@ bool build_chain(FlatPlan const& p, std::vector<uint64_t> const& stage3_bnd, std
                 unit_lines.push_back(line_of);
             }
             for (uint32_t b = 0; b < p.c_nsrows[c]; ++b) {
-                ChainProblem pr{ref(BUF_ABS, outptr[p.c_out_ci[c]] / 8 + uint64_t(b) * ls * rs), 0, left ? ls : rs,
+                ChainProblem pr{ref(BUF_ABS, outptr[p.c_out_ci[c]] / 8 + uint64_t(b) * ls * rs), left ? ls : rs,
                                 left ? rs : ls, left ? 1 : ls, left ? ls : 1, uint32_t(all_lines.size()), 0, 0};
                 for (size_t x = 0; x < units[c].size(); ++x) {
                     const uint32_t u = units[c][x], ms = p.u_ms[u];
@@ -470,7 +469,6 @@ bool build_chain(FlatPlan const& p, std::vector<uint64_t> const& stage3_bnd, std
     uint64_t n_tiles = 0;
     for (auto const& pr : probs) n_tiles += (pr.N + 7) / 8;
     cl.tiles.reserve(n_tiles);
-    cl.block_off.reserve(n_tiles);
     for (auto const& pr : probs) {
         const uint32_t begin = uint32_t(cl.terms.size());
         cost.assign(1, 0);
@@ -521,7 +519,6 @@ bool build_chain(FlatPlan const& p, std::vector<uint64_t> const& stage3_bnd, std
             t.cn = pr.cn;
             std::copy(bounds, bounds + CH_WARPS + 1, t.bounds);
             cl.tiles.push_back(t);
-            cl.block_off.push_back(pr.off);
         }
     }
     // Shares per tile: more warps in flight where the tiles are few (Heisenberg m = 64, 55 tiles:

@@ -185,7 +185,6 @@ struct ChainShape {
 struct ChainList : ChainShape {
     std::vector<DevChainTile> tiles;
     std::vector<DevChainTerm> terms;
-    std::vector<uint64_t> block_off;  // per tile: offset of its H psi output block
 };
 struct ChainDev : ChainShape {
     DevChainTile* tiles = nullptr;
@@ -200,6 +199,7 @@ bool build_chain(FlatPlan const& p, std::vector<uint64_t> const& stage3_bnd, std
 cudaError_t launch_chain(ChainDev const& d, Bases const& bs, cudaStream_t stream);
 
 struct DeviceProgram {
+    uint64_t in_elems = 0, out_elems = 0;  // of the plan's vectors
     GemmList stage1, stage3;
     // the whole plan as chained products (chained): what the native FP64 H psi and the boundary
     // steps run then; the stages stay for the callers that need T or S (emulated and per-block
@@ -330,9 +330,7 @@ struct PipelineProgram {
     uint32_t nparts = 0;
     std::vector<uint64_t> in_cut, out_cut;  // nparts + 1 element offsets each
     std::vector<GemmDev> s1, s3;            // device tile lists per range
-    // chained plans: the tiles of each output range (the records are the program's)
-    bool chained = false;
-    std::vector<ChainDev> ch;
+    bool chained = false;  // the plan's one chained launch between two whole copies instead
 };
 cudaError_t compile_pipeline(FlatPlan const& p, std::vector<uint64_t> const& stage3_bnd,
                              std::vector<uint64_t> const& stage1_bnd, DeviceProgram const& prog, uint32_t nparts,

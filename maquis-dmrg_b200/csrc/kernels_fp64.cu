@@ -1207,6 +1207,8 @@ void compile_program(FlatPlan const& p, std::vector<uint64_t> const& stage3_bnd,
                      std::vector<uint64_t> const& stage1_bnd, std::vector<uint64_t> const& outptr,
                      DeviceProgram& prog, bool stack_rows, bool group_lines) {
     prog = DeviceProgram();
+    prog.in_elems = p.in_size;
+    prog.out_elems = p.out_size;
     const uint32_t nt = p.n_t(), nc = p.n_cohorts();
     std::vector<uint64_t> t_off = t_offsets(p, &prog.t_elems);
     // slack after the last T block: the grouped S build's bulk copies may read one
@@ -1577,25 +1579,12 @@ cudaError_t compile_pipeline(FlatPlan const& p, std::vector<uint64_t> const& sta
                              std::vector<uint64_t> const& stage1_bnd, DeviceProgram const& prog, uint32_t nparts,
                              PipelineProgram& pp) {
     pp = PipelineProgram();
+    pp.chained = prog.chained;
+    if (pp.chained) return cudaSuccess;  // one launch, no ranges
     pp.nparts = nparts;
     std::vector<uint64_t> in_off(p.in_off.begin(), p.in_off.end()), out_off(p.out_off.begin(), p.out_off.end());
     pp.in_cut = cut_ranges(in_off, p.in_size, nparts);
     pp.out_cut = cut_ranges(out_off, p.out_size, nparts);
-    if (prog.chained) {
-        pp.chained = true;
-        for (uint32_t q = 0; q < nparts; ++q) {
-            std::vector<DevChainTile> tiles;
-            for (size_t i = 0; i < prog.chain.tiles.size(); ++i)
-                if (prog.chain.block_off[i] >= pp.out_cut[q] && prog.chain.block_off[i] < pp.out_cut[q + 1])
-                    tiles.push_back(prog.chain.tiles[i]);
-            ChainDev d = prog.d_chain;
-            d.n = uint32_t(tiles.size());
-            const cudaError_t e = up(tiles, &d.tiles);
-            pp.ch.push_back(d);
-            if (e != cudaSuccess) return e;
-        }
-        return cudaSuccess;
-    }
     const std::vector<uint64_t> t_off = t_offsets(p, nullptr), s_off = s_offsets(p, nullptr);
     pp.s1.resize(nparts);
     pp.s3.resize(nparts);
@@ -1623,7 +1612,6 @@ cudaError_t compile_pipeline(FlatPlan const& p, std::vector<uint64_t> const& sta
 void free_pipeline(PipelineProgram& pp) {
     for (auto& g : pp.s1) free_gemm(g);
     for (auto& g : pp.s3) free_gemm(g);
-    for (auto& c : pp.ch) cudaFree(c.tiles);
     pp = PipelineProgram();
 }
 
@@ -1637,6 +1625,16 @@ cudaError_t run_pipeline(DeviceProgram const& prog, PipelineProgram const& pp, c
     bs.b[BUF_T] = reinterpret_cast<uint64_t>(T);
     bs.b[BUF_S] = reinterpret_cast<uint64_t>(S);
     cudaError_t e;
+    if (pp.chained) {
+        // Chained products read all of x for every output, so nothing overlaps the copy in, and a
+        // launch per output range to overlap the copy out costs more than it hides: the ranges
+        // are too short to fill the chip (Hubbard L = 32, m = 480, 0.96 MB each way: 115 us by
+        // four ranges, 107 by the stages in ranges, 70 in sequence).
+        if ((e = cudaMemcpyAsync(xd, x_host, prog.in_elems * sizeof(double), cudaMemcpyHostToDevice, s)) != cudaSuccess)
+            return e;
+        if ((e = launch_chain(prog.d_chain, bs, s)) != cudaSuccess) return e;
+        return cudaMemcpyAsync(y_host, yd, prog.out_elems * sizeof(double), cudaMemcpyDeviceToHost, s);
+    }
     // the copies start after the work already queued on the caller's stream
     if ((e = cudaEventRecord(ev[0], s)) != cudaSuccess) return e;
     if ((e = cudaStreamWaitEvent(c, ev[0], 0)) != cudaSuccess) return e;
@@ -1649,20 +1647,15 @@ cudaError_t run_pipeline(DeviceProgram const& prog, PipelineProgram const& pp, c
     }
     for (uint32_t q = 0; q < np; ++q) {
         if ((e = cudaStreamWaitEvent(s, ev[1 + q], 0)) != cudaSuccess) return e;
-        if (pp.chained) continue;  // every output range needs the whole input
         GemmDev g = pp.s1[q];
         g.var = prog.var1;
         if ((e = launch_gemm(g, bs, s)) != cudaSuccess) return e;
     }
-    if (!pp.chained && (e = run_sbuild(prog, T, S, s)) != cudaSuccess) return e;
+    if ((e = run_sbuild(prog, T, S, s)) != cudaSuccess) return e;
     for (uint32_t q = 0; q < np; ++q) {
-        if (pp.chained) {
-            if ((e = launch_chain(pp.ch[q], bs, s)) != cudaSuccess) return e;
-        } else {
-            GemmDev g = pp.s3[q];
-            g.var = prog.var3;
-            if ((e = launch_gemm(g, bs, s)) != cudaSuccess) return e;
-        }
+        GemmDev g = pp.s3[q];
+        g.var = prog.var3;
+        if ((e = launch_gemm(g, bs, s)) != cudaSuccess) return e;
         if ((e = cudaEventRecord(ev[1 + np + q], s)) != cudaSuccess) return e;
         if ((e = cudaStreamWaitEvent(c, ev[1 + np + q], 0)) != cudaSuccess) return e;
         const uint64_t n = pp.out_cut[q + 1] - pp.out_cut[q];

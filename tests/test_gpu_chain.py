@@ -98,7 +98,7 @@ def test_chain_matches_oracle_and_stages(name, L, m, i, chained):
     y = yd.cpu().numpy()
     assert np.all(np.isnan(y[~mask]))  # the padding of y is left untouched
     assert _rel(y[mask], ref[mask]) <= TOL
-    # host buffers run the same tiles by output range
+    # host buffers run the same launch between two copies
     xh = torch.from_numpy(x.copy()).pin_memory()
     yh = torch.zeros_like(xh).pin_memory()
     plan.hpsi_host(xh.data_ptr(), yh.data_ptr())
