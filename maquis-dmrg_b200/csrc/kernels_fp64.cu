@@ -114,7 +114,7 @@ struct CopyStream {
     bool rowmajor;
 };
 
-template <int ROWS, int BK_, int NTHREADS, int LD>
+template <int ROWS, int BK_, int NTHREADS, int LD, bool HALVES>
 __device__ __forceinline__ void issue_copies(double* tile, CopyStream& cs, uint32_t krem) {
     constexpr int NC = ROWS * BK_ / NTHREADS;
     if (BK_ < 16) {
@@ -138,7 +138,7 @@ __device__ __forceinline__ void issue_copies(double* tile, CopyStream& cs, uint3
                 for (int j = 0; j < NC; ++j, p += cs.jstride)
                     cp_async8_all(&tile[(cs.kt + j * KJ) * LD + (cs.r ^ ((t0 + ((j * KJ) >> 2)) & 3u))], p);
             } else {
-                const uint32_t kend = krem > uint32_t(BK_ / 2) ? BK_ : BK_ / 2;
+                const uint32_t kend = !HALVES || krem > uint32_t(BK_ / 2) ? BK_ : BK_ / 2;
 #pragma unroll
                 for (int j = 0; j < NC; ++j, p += cs.jstride) {
                     const uint32_t k = cs.kt + j * KJ;
@@ -158,7 +158,7 @@ __device__ __forceinline__ void issue_copies(double* tile, CopyStream& cs, uint3
 #pragma unroll
             for (int j = 0; j < NC; ++j, p += cs.jstride)
                 if ((cs.mask >> j) & 1u) cp_async8_all(dst + j * RJ, p);
-        } else if (cs.kt < (krem > uint32_t(BK_ / 2) ? BK_ : BK_ / 2)) {
+        } else if (!HALVES || cs.kt < (krem > uint32_t(BK_ / 2) ? BK_ : BK_ / 2)) {
 #pragma unroll
             for (int j = 0; j < NC; ++j, p += cs.jstride)
                 if ((cs.mask >> j) & 1u) cp_async8(dst + j * RJ, reinterpret_cast<const double*>(kok ? p : cs.safe), kok);
@@ -209,7 +209,7 @@ struct LoadCursor {
     bool valid;
 };
 
-template <int BM_, int BN_, int BK_, int STAGES, int MINB, int NTHREADS, int WARPS_M>
+template <int BM_, int BN_, int BK_, int STAGES, int MINB, int NTHREADS, int WARPS_M, bool HALVES = true>
 __global__ void __launch_bounds__(NTHREADS, MINB) gemm_f64_grouped(const DevProb* __restrict__ probs,
                                                                    const DevSeg* __restrict__ segs,
                                                                    const DevTile* __restrict__ tiles, uint32_t n_tiles,
@@ -288,8 +288,8 @@ __global__ void __launch_bounds__(NTHREADS, MINB) gemm_f64_grouped(const DevProb
         uint32_t rows = 0;
         if (L.seg < L.seg_end) {  // an empty tile issues no copies
             rows = min(L.krem, uint32_t(BK_));
-            issue_copies<BM_, BK_, NTHREADS, pitch<BM_>()>(&As[slot][0][0], ca, L.krem);
-            issue_copies<BN_, BK_, NTHREADS, pitch<BN_>()>(&Bs[slot][0][0], cb, L.krem);
+            issue_copies<BM_, BK_, NTHREADS, pitch<BM_>(), HALVES>(&As[slot][0][0], ca, L.krem);
+            issue_copies<BN_, BK_, NTHREADS, pitch<BN_>(), HALVES>(&Bs[slot][0][0], cb, L.krem);
             if (L.krem > uint32_t(BK_)) {
                 L.krem -= BK_;
                 return rows;
@@ -335,10 +335,10 @@ __global__ void __launch_bounds__(NTHREADS, MINB) gemm_f64_grouped(const DevProb
             cp_async_commit();
             cp_async_wait<STAGES - 1>();
             __syncthreads();
-            // the second half of a stage that holds at most half its K rows is not multiplied, nor
-            // tiles of warps outside the problem; unrolled forms keep the fragment reads ahead of the
-            // products (a condition per K step of four, or a form per count of them, costs more
-            // than it saves where a CTA has its SM to itself)
+            // the second half of a stage that holds at most half its K rows is not multiplied
+            // (HALVES), nor tiles of warps outside the problem; unrolled forms keep the fragment
+            // reads ahead of the products (a condition per K step of four, or a form per count of
+            // them, costs more than it saves where a CTA has its SM to itself)
             if (inside) {
                 auto product = [&](auto steps) {
                     constexpr int KS = decltype(steps)::value;
@@ -355,8 +355,8 @@ __global__ void __launch_bounds__(NTHREADS, MINB) gemm_f64_grouped(const DevProb
                             for (int j = 0; j < NJ; ++j) dmma(acc[i][j][0], acc[i][j][1], a[i], b[j]);
                     }
                 };
-                if (kn > uint32_t(BK_ / 2)) product(std::integral_constant<int, BK_ / 4>());
-                else if (kn) product(std::integral_constant<int, BK_ / 8>());
+                if (HALVES ? kn > uint32_t(BK_ / 2) : kn > 0) product(std::integral_constant<int, BK_ / 4>());
+                else if (HALVES && kn) product(std::integral_constant<int, BK_ / 8>());
             }
             __syncthreads();
             slot = (slot + 1) % STAGES;
@@ -1739,8 +1739,12 @@ struct GemmVariant {
     int tile_class;  // which tile list it runs on
     int threads;     // CTA size
 };
+// Variant 0 multiplies whole stages: it is the one of plans too small to tune, whose CTAs have an
+// SM to themselves, and there the second form and its branch cost more than the skipped products
+// (H psi of Heisenberg m = 240, 300 19.9, 21.5 us with halves, 19.6, 20.9 without; Hubbard m = 1600,
+// full of short stages and tuned to others, 143 us with and 147 without).
 const GemmVariant kVariants[N_GEMM_VARIANTS] = {
-    {gemm_f64_grouped<32, 64, 16, 2, 4, 128, 2>, "tile32x64_k16_stages2_ctas4", 0, 128},
+    {gemm_f64_grouped<32, 64, 16, 2, 4, 128, 2, false>, "tile32x64_k16_stages2_ctas4", 0, 128},
     {gemm_f64_grouped<32, 64, 16, 3, 4, 128, 2>, "tile32x64_k16_stages3_ctas4", 0, 128},
     {gemm_f64_grouped<32, 64, 16, 2, 5, 128, 2>, "tile32x64_k16_stages2_ctas5", 0, 128},
     {gemm_f64_grouped<32, 64, 16, 3, 5, 128, 2>, "tile32x64_k16_stages3_ctas5", 0, 128},
