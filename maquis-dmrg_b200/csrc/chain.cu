@@ -291,7 +291,7 @@ bool chain_sizes(FlatPlan const& p) {
     }
     for (uint32_t ob = 0; p.kind == KIND_HPSI && ob < p.out_rows.size(); ++ob)
         if (!written[ob] && !problem(p.out_rows[ob], p.out_cols[ob])) return false;
-    return tiles <= 148 * 16;
+    return tiles <= 16 * B200_SMS;
 }
 
 }  // namespace
@@ -529,7 +529,7 @@ bool build_chain(FlatPlan const& p, std::vector<uint64_t> const& stage3_bnd, std
         cl = ChainList();
         return false;
     }
-    cl.split = cl.tiles.size() < 148 * 6 ? 4 : cl.tiles.size() < 148 * 10 ? 2 : 1;
+    cl.split = cl.tiles.size() < 6 * B200_SMS ? 4 : cl.tiles.size() < 10 * B200_SMS ? 2 : 1;
     return true;
 }
 

@@ -130,6 +130,10 @@ struct DevArray {
     size_t n = 0;
 };
 
+// SMs of the GPU this is written for.  Rules that decide how a plan's sums are ordered count
+// these and not the device's own, so that a plan gives the same bits on a partition of one.
+constexpr uint32_t B200_SMS = 148;
+
 // tile classes of the grouped GEMM: 0 = 32 x 64 tiles with 16-deep K steps,
 // 1 = 16 x 64 with 8-deep steps, 2 = 64 x 64 with 16-deep steps, 3 = 16 x 64
 // with 16-deep steps

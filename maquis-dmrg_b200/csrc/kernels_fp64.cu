@@ -1101,7 +1101,7 @@ namespace {
 uint32_t split_target(GemmList const& gl) {
     uint64_t total = 0;
     for (auto const& t : gl.tiles) total += t.nsteps;
-    return uint32_t(std::max<uint64_t>(48, total / (2 * 4 * 148)));
+    return uint32_t(std::max<uint64_t>(48, total / (2 * 4 * B200_SMS)));
 }
 
 // `gl` with K ranges of more than `target` steps cut into parts, a function of the problem and
@@ -1414,7 +1414,7 @@ void compile_program(FlatPlan const& p, std::vector<uint64_t> const& stage3_bnd,
     if (stack_rows && group_lines && mode == 0 && ug_units.empty())
         prog.chained = prog.chain_built = build_chain(p, stage3_bnd, stage1_bnd, outptr, prog.chain);
     // ---- stage 3 with long K ranges split ----
-    if (stack_rows && group_lines && g3.tiles.size() < 4 * 4 * 148) {
+    if (stack_rows && group_lines && g3.tiles.size() < 4 * 4 * B200_SMS) {
         prog.split_steps = split_target(g3);
         prog.own3 = split_list(g3, prog.split_steps, prog.stage3f);
     }
@@ -1692,7 +1692,7 @@ double calibrate_fp64_tflops() {
 
 void gemm_split_long(GemmList& gl) {
     GemmList cut;
-    if (gl.tiles.size() < 4 * 4 * 148 && split_list(gl, split_target(gl), cut)) gl = std::move(cut);
+    if (gl.tiles.size() < 4 * 4 * B200_SMS && split_list(gl, split_target(gl), cut)) gl = std::move(cut);
 }
 
 cudaError_t upload_gemm(GemmList const& gl, GemmDev& d) {
@@ -1811,7 +1811,7 @@ cudaError_t launch_variant(int v, const DevProb* p, const DevSeg* sg, const DevT
 
 // 64 x 64 tiles at three CTAs per SM where they fill the chip twice (SU2U1 L=16 m=512 stage 1,
 // 472 us against 536 for 32 x 64; on shorter lists the smaller tiles balance better)
-int gemm_default_variant(GemmList const& gl) { return gl.tiles_cls[2].size() >= 2 * 3 * 148 ? 6 : 0; }
+int gemm_default_variant(GemmList const& gl) { return gl.tiles_cls[2].size() >= 2 * 3 * B200_SMS ? 6 : 0; }
 
 const char* gemm_variant_name(int v) { return (v >= 0 && v < N_GEMM_VARIANTS) ? kVariants[v].name : "?"; }
 
@@ -1930,7 +1930,7 @@ int device_sm_count() {
     int dev = 0, n = 0;
     cudaGetDevice(&dev);
     cudaDeviceGetAttribute(&n, cudaDevAttrMultiProcessorCount, dev);
-    return n > 0 ? n : 148;
+    return n > 0 ? n : int(B200_SMS);
 }
 
 cudaError_t run_stages12(DeviceProgram const& prog, uint64_t in, uint64_t out, double* T, double* S,
