@@ -209,7 +209,8 @@ struct LoadCursor {
     bool valid;
 };
 
-template <int BM_, int BN_, int BK_, int STAGES, int MINB, int NTHREADS, int WARPS_M, bool HALVES = true>
+template <int BM_, int BN_, int BK_, int STAGES, int MINB, int NTHREADS, int WARPS_M, bool HALVES = true,
+          bool LEAN = false>
 __global__ void __launch_bounds__(NTHREADS, MINB) gemm_f64_grouped(const DevProb* __restrict__ probs,
                                                                    const DevSeg* __restrict__ segs,
                                                                    const DevTile* __restrict__ tiles, uint32_t n_tiles,
@@ -230,7 +231,7 @@ __global__ void __launch_bounds__(NTHREADS, MINB) gemm_f64_grouped(const DevProb
     const int tid = threadIdx.x;
     // one value per warp also to the compiler: branches on the warp's place need no reconvergence
     // (Heisenberg m = 230 to 400 19.2 to 26.8 us without, 18.8 to 26.4 with)
-    const int lane = tid & 31, warp = __shfl_sync(0xffffffffu, tid >> 5, 0);
+    const int lane = tid & 31, warp = LEAN ? tid >> 5 : __shfl_sync(0xffffffffu, tid >> 5, 0);
     const int wm = (warp % WARPS_M) * WM, wn = (warp / WARPS_M) * WN;
     const int g = lane >> 2, q = lane & 3;
 
@@ -326,7 +327,7 @@ __global__ void __launch_bounds__(NTHREADS, MINB) gemm_f64_grouped(const DevProb
         const DevTile tl = tiles[ti];
         const DevProb& pr = probs[tl.prob];
         const uint32_t M = pr.M, N = pr.N;
-        const bool inside = tl.m0 + wm < M && tl.n0 + wn < N;  // any of this warp's tile
+        const bool inside = LEAN || (tl.m0 + wm < M && tl.n0 + wn < N);  // any of this warp's tile
         for (uint32_t st = 0; st < tl.nsteps; ++st) {
             const uint32_t kn = held[0];
             held[STAGES - 1] = issue((slot + STAGES - 1) % STAGES);
@@ -355,14 +356,16 @@ __global__ void __launch_bounds__(NTHREADS, MINB) gemm_f64_grouped(const DevProb
                             for (int j = 0; j < NJ; ++j) dmma(acc[i][j][0], acc[i][j][1], a[i], b[j]);
                     }
                 };
-                if (HALVES ? kn > uint32_t(BK_ / 2) : kn > 0) product(std::integral_constant<int, BK_ / 4>());
+                if (LEAN || (HALVES ? kn > uint32_t(BK_ / 2) : kn > 0)) product(std::integral_constant<int, BK_ / 4>());
                 else if (HALVES && kn) product(std::integral_constant<int, BK_ / 8>());
             }
             __syncthreads();
             slot = (slot + 1) % STAGES;
         }
         // epilogue (the next tile's first steps are already in flight); an empty tile multiplied
-        // nothing and stores zeros
+        // nothing (LEAN: what it found) and stores zeros
+        bool empty = LEAN;
+        for (uint32_t sg = pr.seg_begin; LEAN && sg < pr.seg_end; ++sg) empty = empty && segs[sg].K == 0;
         if (pr.split != DevProb::NO_SPLIT) {
             const DevSplit sp = split.tab[pr.split];
             const uint64_t mn = uint64_t(M) * N;
@@ -425,7 +428,7 @@ __global__ void __launch_bounds__(NTHREADS, MINB) gemm_f64_grouped(const DevProb
 #pragma unroll
                 for (int e = 0; e < 2; ++e) {
                     uint32_t c = tl.n0 + wn + j * 8 + q * 2 + e;
-                    if (r < M && c < N) crow[c * ld] = acc[i][j][e];
+                    if (r < M && c < N) crow[c * ld] = empty ? 0.0 : acc[i][j][e];
                     acc[i][j][e] = 0.0;
                 }
         }
@@ -1743,13 +1746,16 @@ struct GemmVariant {
 // SM to themselves, and there the second form and its branch cost more than the skipped products
 // (H psi of Heisenberg m = 240, 300 19.9, 21.5 us with halves, 19.6, 20.9 without; Hubbard m = 1600,
 // full of short stages and tuned to others, 143 us with and 147 without).
+// Variant 5 has 64 registers a thread for eight CTAs per SM: it goes without the counts of the
+// stages in flight and the test of the warp's place (LEAN), which spilled 80 bytes into every K
+// step (4096^3 6.1 TFLOP/s; Heisenberg m = 400 33.5 us on stage 3, 23.5 LEAN).
 const GemmVariant kVariants[N_GEMM_VARIANTS] = {
     {gemm_f64_grouped<32, 64, 16, 2, 4, 128, 2, false>, "tile32x64_k16_stages2_ctas4", 0, 128},
     {gemm_f64_grouped<32, 64, 16, 3, 4, 128, 2>, "tile32x64_k16_stages3_ctas4", 0, 128},
     {gemm_f64_grouped<32, 64, 16, 2, 5, 128, 2>, "tile32x64_k16_stages2_ctas5", 0, 128},
     {gemm_f64_grouped<32, 64, 16, 3, 5, 128, 2>, "tile32x64_k16_stages3_ctas5", 0, 128},
     {gemm_f64_grouped<16, 64, 8, 3, 6, 128, 1>, "tile16x64_k8_stages3_ctas6", 1, 128},
-    {gemm_f64_grouped<16, 64, 8, 4, 8, 128, 1>, "tile16x64_k8_stages4_ctas8", 1, 128},
+    {gemm_f64_grouped<16, 64, 8, 4, 8, 128, 1, false, true>, "tile16x64_k8_stages4_ctas8", 1, 128},
     {gemm_f64_grouped<64, 64, 16, 2, 3, 128, 2>, "tile64x64_k16_stages2_ctas3", 2, 128},
     {gemm_f64_grouped<64, 64, 16, 2, 2, 128, 2>, "tile64x64_k16_stages2_ctas2", 2, 128},
     {gemm_f64_grouped<16, 64, 16, 2, 8, 64, 1>, "tile16x64_k16_warps2_stages2_ctas8", 3, 64},
